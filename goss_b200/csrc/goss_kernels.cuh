@@ -121,11 +121,46 @@ __device__ __forceinline__ void load_field(const double* __restrict__ fp, uint64
         F[k] = (k < M::num_field_params) ? T(fp[k * ld + node]) : T(0);
 }
 
-// GRL increment of one state, FP64: the reference expression
+// GRL increment of one state, FP64, in the reference's own expression
 // b/a*(exp(a*h) - 1.0) or b*h (GRL1.h:80-83)
-__device__ __forceinline__ double grl_increment(double a, double b, double h, double delta)
+__device__ __forceinline__ double grl_increment_printed(double a, double b, double h, double delta)
 {
     return (fabs(a) > delta) ? b / a * (exp(a * h) - 1.0) : b * h;
+}
+
+// coefficients up to this size take the Euler increment whatever delta is:
+// their reciprocal could overflow
+constexpr double kGrlTiny = 0x1p-1000;
+
+// The same expression for N states at once, with branch-free arithmetic.
+// e^x - 1 keeps the rounding of e^x to a double (its cancellation is part of
+// the reference's results: the exact (e^x - 1)/x, cheaper and more accurate,
+// differed from them by up to 1.4e-10 of V through an upstroke).  For
+// |x| < 1/8 -- gates slower than 8 h, nearly all states of a cardiac model at
+// its usual step -- e^x is 1 + x phi1(x) in one FMA over a polynomial, beyond
+// that f64_exp, under one branch for the N states so that their polynomials
+// and reciprocals overlap.
+template <int N>
+__device__ __forceinline__ void grl_increments(const double* a, const double* b, double h, double delta, double* inc)
+{
+    double x[N], e[N];
+    int far = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        x[i] = a[i] * h;
+        e[i] = fma(x[i], models::f64_phi1_small(x[i]), 1.0);
+        inc[i] = b[i] * models::f64_rcp(a[i]);
+        far = max(far, __double2hiint(x[i]) & 0x7fffffff);
+    }
+    if (far >= 0x3fc00000) {  // |x| >= 1/8, infinite or NaN
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if ((__double2hiint(x[i]) & 0x7fffffff) >= 0x3fc00000)
+                e[i] = models::f64_exp(x[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        inc[i] = fabs(a[i]) > delta ? inc[i] * (e[i] - 1.0) : b[i] * h;
 }
 
 // GRL increment of one state, FP32: b*h*phi1(a*h), algebraically identical
@@ -138,12 +173,20 @@ __device__ __forceinline__ float grl_increment(float a, float b, float h, float 
     return b * h * phi1f(a * h);
 }
 
+template <int N>
+__device__ __forceinline__ void grl_increments(const float* a, const float* b, float h, float delta, float* inc)
+{
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        inc[i] = grl_increment(a[i], b[i], h, delta);
+}
+
 // RL increment of one state (RL1.h:68-77): the exponential form for the model's
 // linear-term states whatever the coefficient (the reference divides by it),
 // the Euler increment otherwise
 __device__ __forceinline__ double rl_increment(bool linear, double a, double b, double h)
 {
-    return linear ? b / a * (exp(a * h) - 1.0) : b * h;
+    return linear ? models::f64_div(b, a) * (models::f64_exp(a * h) - 1.0) : b * h;
 }
 __device__ __forceinline__ float rl_increment(bool linear, float a, float b, float h)
 {
@@ -250,6 +293,30 @@ struct NodeIO {
 // reference over 10^5 TP06 GRL1 steps.  Printed = true takes the programs in
 // the printed operation order of the model (one exp per occurrence, divisions
 // as written), the arithmetic of the reference's own generated code.
+// Split FP64 programs run on models::F64, a double whose division,
+// exponentials and square root have no branches (goss_device_math.cuh).
+template <typename T>
+struct SplitScalar {
+    using type = T;
+};
+template <>
+struct SplitScalar<double> {
+    using type = models::F64;
+};
+template <typename T>
+using split_t = typename SplitScalar<T>::type;
+// a double array as the split programs' scalars, and the reverse
+template <typename T>
+__device__ __forceinline__ const split_t<T>* as_split(const T* p)
+{
+    return reinterpret_cast<const split_t<T>*>(p);
+}
+template <typename T>
+__device__ __forceinline__ split_t<T>* as_split(T* p)
+{
+    return reinterpret_cast<split_t<T>*>(p);
+}
+
 template <class M, typename T, bool Printed = false>
 __device__ __forceinline__ void model_linearized(const T* y, double t, const T* P, const double* PD, const T* F,
                                                  T* lin, T* rhs)
@@ -257,12 +324,40 @@ __device__ __forceinline__ void model_linearized(const T* y, double t, const T* 
     if constexpr (Printed)
         M::template linearized<T>(y, t, P, PD, F, lin, rhs);
     else
-        M::template linearized_split<T>(y, t, P, PD, F, lin, rhs);
+        M::template linearized_split<split_t<T>>(as_split(y), t, as_split(P), PD, as_split(F), as_split(lin),
+                                                 as_split(rhs));
 }
 template <class M, typename T>
 __device__ __forceinline__ void model_rhs(const T* y, double t, const T* P, const double* PD, const T* F, T* f)
 {
-    M::template rhs_split<T>(y, t, P, PD, F, f);
+    M::template rhs_split<split_t<T>>(as_split(y), t, as_split(P), PD, as_split(F), as_split(f));
+}
+
+// the threshold below which a coefficient takes the Euler increment
+__device__ __forceinline__ double grl_delta(double delta) { return fmax(delta, kGrlTiny); }
+__device__ __forceinline__ float grl_delta(float delta) { return delta; }
+
+// put(y[i], i, GRL increment of state i) for every state, in FP64 four states
+// at a time
+template <int n, typename T, class Put>
+__device__ __forceinline__ void grl_apply(Acc<T>* y, const T* lin, const T* rhs, T h, T delta, Put&& put)
+{
+    constexpr int N = sizeof(T) == 4 ? 1 : 4;
+    T inc[N];
+#pragma unroll
+    for (int i = 0; i + N <= n; i += N) {
+        grl_increments<N>(lin + i, rhs + i, h, delta, inc);
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            put(y[i + k], i + k, inc[k]);
+    }
+    if constexpr (n % N != 0) {
+        constexpr int i = n - n % N;
+        grl_increments<n % N>(lin + i, rhs + i, h, delta, inc);
+#pragma unroll
+        for (int k = 0; k < n % N; ++k)
+            put(y[i + k], i + k, inc[k]);
+    }
 }
 
 // One internal step of an explicit solver at time lt with step ldt, in place
@@ -289,58 +384,52 @@ __device__ __forceinline__ void explicit_step(Acc<T>* y, const double lt, const 
     } else if constexpr (S == Explicit::RK4) {
         // RK4.cpp:79-98 with RK4::axpy (RK4.h:70-74); the weighted sum is
         // accumulated in the order k1 + 2 k2 + 2 k3 + k4 of the reference.
-        T k[n], sum[n], tmp[n];
-        model_rhs<M, T>(yt, lt, P, PD, F, k);
+        // FP64: one copy of the right-hand side for the four stages (four
+        // copies do not stay in the instruction cache: TP06, 262,144 nodes x
+        // 100 steps 16.7 -> 12.2 ms; FP32, with a third of the instructions
+        // per evaluation, 2.49 -> 2.66 ms, stays unrolled).
+        T sum[n];
+#pragma unroll(sizeof(T) == 4 ? 4 : 1)
+        for (int st = 0; st < 4; ++st) {
+            T k[n];
+            model_rhs<M, T>(yt, st == 0 ? lt : st == 3 ? lt + ldt : lt + 0.5 * ldt, P, PD, F, k);
+            const T w = st == 1 || st == 2 ? T(2.0) : T(1.0), c = st == 2 ? h : hh;
 #pragma unroll
-        for (int i = 0; i < n; ++i) {
-            sum[i] = k[i];
-            tmp[i] = y[i].plus(hh * k[i]);
+            for (int i = 0; i < n; ++i) {
+                sum[i] = st == 0 ? k[i] : sum[i] + w * k[i];
+                yt[i] = y[i].plus(c * k[i]);
+            }
         }
-        model_rhs<M, T>(tmp, lt + 0.5 * ldt, P, PD, F, k);
 #pragma unroll
-        for (int i = 0; i < n; ++i) {
-            sum[i] = sum[i] + T(2.0) * k[i];
-            tmp[i] = y[i].plus(hh * k[i]);
-        }
-        model_rhs<M, T>(tmp, lt + 0.5 * ldt, P, PD, F, k);
-#pragma unroll
-        for (int i = 0; i < n; ++i) {
-            sum[i] = sum[i] + T(2.0) * k[i];
-            tmp[i] = y[i].plus(h * k[i]);
-        }
-        model_rhs<M, T>(tmp, lt + ldt, P, PD, F, k);
-#pragma unroll
-        for (int i = 0; i < n; ++i) {
-            sum[i] = sum[i] + k[i];
-            y[i].add(h * sum[i] / T(6.0));
-        }
+        for (int i = 0; i < n; ++i)
+            y[i].add(T(split_t<T>(h * sum[i]) / split_t<T>(6.0)));
     } else if constexpr (S == Explicit::GRL1) {
         // GRL1.h:72-84
         T lin[n], rhs[n];
         model_linearized<M, T>(yt, lt, P, PD, F, lin, rhs);
-#pragma unroll
-        for (int i = 0; i < n; ++i)
-            y[i].add(grl_increment(lin[i], rhs[i], h, delta));
+        grl_apply<n>(y, lin, rhs, h, grl_delta(delta), [](Acc<T>& v, int, T d) { v.add(d); });
     } else if constexpr (S == Explicit::GRL1Printed) {
         // GRL1.h:72-84 over the printed model program
         T lin[n], rhs[n];
         model_linearized<M, T, true>(yt, lt, P, PD, F, lin, rhs);
 #pragma unroll
         for (int i = 0; i < n; ++i)
-            y[i].add(grl_increment(lin[i], rhs[i], h, delta));
+            y[i].add(grl_increment_printed(lin[i], rhs[i], h, delta));
     } else if constexpr (S == Explicit::GRL2) {
         // GRL2: GRL2.cpp:78-82.  The reference's branch threshold is a
         // self-initialised local (GRL2.cpp:67) whose -O3 build behaves as 0:
         // the exponential form is used whenever the linear term is non-zero.
-        T lin[n], rhs[n], y2[n];
-        model_linearized<M, T>(yt, lt, P, PD, F, lin, rhs);
-#pragma unroll
-        for (int i = 0; i < n; ++i)
-            y2[i] = y[i].plus(grl_increment(lin[i], rhs[i], hh, T(0)));
-        model_linearized<M, T>(y2, lt, P, PD, F, lin, rhs);
-#pragma unroll
-        for (int i = 0; i < n; ++i)
-            y[i].add(grl_increment(lin[i], rhs[i], h, T(0)));
+        // FP64: one copy of the linearised model for both evaluations, as in
+        // RK4 (9.4 -> 8.2 ms; FP32 1.82 -> 1.92 ms, stays unrolled).
+#pragma unroll(sizeof(T) == 4 ? 2 : 1)
+        for (int st = 0; st < 2; ++st) {
+            T lin[n], rhs[n];
+            model_linearized<M, T>(yt, lt, P, PD, F, lin, rhs);
+            if (st == 0)
+                grl_apply<n>(y, lin, rhs, hh, grl_delta(T(0)), [&](Acc<T>& v, int i, T d) { yt[i] = v.plus(d); });
+            else
+                grl_apply<n>(y, lin, rhs, h, grl_delta(T(0)), [](Acc<T>& v, int, T d) { v.add(d); });
+        }
     } else if constexpr (S == Explicit::RL1) {
         // RL1.h:68-77
         T lin[n], rhs[n];
@@ -351,27 +440,34 @@ __device__ __forceinline__ void explicit_step(Acc<T>* y, const double lt, const 
     } else if constexpr (S == Explicit::RL2) {
         // RL2.cpp:78-83: a half step to y2 linearised at y, then the full step
         // from y linearised at y2, both at time lt
-        T lin[n], rhs[n], y2[n];
-        model_linearized<M, T>(yt, lt, P, PD, F, lin, rhs);
+#pragma unroll(sizeof(T) == 4 ? 2 : 1)
+        for (int st = 0; st < 2; ++st) {
+            T lin[n], rhs[n];
+            model_linearized<M, T>(yt, lt, P, PD, F, lin, rhs);
 #pragma unroll
-        for (int i = 0; i < n; ++i)
-            y2[i] = y[i].plus(rl_increment(M::linear_term(i), lin[i], rhs[i], hh));
-        model_linearized<M, T>(y2, lt, P, PD, F, lin, rhs);
-#pragma unroll
-        for (int i = 0; i < n; ++i)
-            y[i].add(rl_increment(M::linear_term(i), lin[i], rhs[i], h));
+            for (int i = 0; i < n; ++i) {
+                const T d = rl_increment(M::linear_term(i), lin[i], rhs[i], st == 0 ? hh : h);
+                if (st == 0)
+                    yt[i] = y[i].plus(d);
+                else
+                    y[i].add(d);
+            }
+        }
     } else {
         // RK2: RK2.cpp:78-89 with RK2::axpy (RK2.h:70-74), the midpoint rule
         static_assert(S == Explicit::RK2, "unhandled explicit solver");
-        T k[n], tmp[n];
-        model_rhs<M, T>(yt, lt, P, PD, F, k);
+#pragma unroll(sizeof(T) == 4 ? 2 : 1)
+        for (int st = 0; st < 2; ++st) {
+            T k[n];
+            model_rhs<M, T>(yt, st == 0 ? lt : lt + 0.5 * ldt, P, PD, F, k);
 #pragma unroll
-        for (int i = 0; i < n; ++i)
-            tmp[i] = y[i].plus(hh * k[i]);
-        model_rhs<M, T>(tmp, lt + 0.5 * ldt, P, PD, F, k);
-#pragma unroll
-        for (int i = 0; i < n; ++i)
-            y[i].add(h * k[i]);
+            for (int i = 0; i < n; ++i) {
+                if (st == 0)
+                    yt[i] = y[i].plus(hh * k[i]);
+                else
+                    y[i].add(h * k[i]);
+            }
+        }
     }
 }
 
@@ -445,26 +541,22 @@ __device__ __forceinline__ void explicit_node_from(const NodeIO& a, uint32_t nod
 }
 
 // Resident blocks of 128 threads per SM the explicit kernels are compiled for
-// (register cap 65536 / (128 * blocks)).  FP64: 3 for the one-evaluation
-// steps (170 registers), 4 for those with two or more evaluations (128
-// registers): measured on B200 (TP06, 1,048,576 nodes, four fields) against
-// the uncapped 255 registers, GRL1 3.55e9 -> 4.10e9 cell-steps/s (4: 3.90e9),
-// GRL2 1.09e9 -> 1.82e9 (3: 1.57e9); more warps hide the FP64 latencies
-// better than the spills cost.  FP32: uncapped (150 registers for TP06 GRL1,
-// 3 blocks per SM); capping it at 128 registers measured 2.77e10 against
-// 2.91e10 cell-steps/s.
+// (register cap 65536 / (128 * blocks)).  FP64: 3 (168 registers): measured on
+// B200 (TP06, 262,144 nodes x 100 steps, four fields), blocks 2 / 3 / 4: GRL1
+// 3.91 / 3.73 / 3.96 ms, GRL2 8.23 / 8.24 / 9.26, RK4 12.4 / 12.2 / 12.9; more
+// warps hide the FP64 latencies better than the spills cost up to there.
+// FP32: uncapped (150 registers for TP06 GRL1, 3 blocks per SM); capping it at
+// 128 registers measured 2.77e10 against 2.91e10 cell-steps/s.
 #ifndef GOSS_EXPLICIT_MIN_BLOCKS_FP32
 #define GOSS_EXPLICIT_MIN_BLOCKS_FP32 1
 #endif
-template <typename T, Explicit S>
+template <typename T>
 struct ExplicitMinBlocks {
-    static constexpr bool one_eval = S == Explicit::Euler || S == Explicit::GRL1 || S == Explicit::RL1 ||
-                                     S == Explicit::GRL1Printed;
-    static constexpr int value = sizeof(T) == 4 ? GOSS_EXPLICIT_MIN_BLOCKS_FP32 : (one_eval ? 3 : 4);
+    static constexpr int value = sizeof(T) == 4 ? GOSS_EXPLICIT_MIN_BLOCKS_FP32 : 3;
 };
 
 template <class M, typename T, Explicit S>
-__global__ void __launch_bounds__(128, (ExplicitMinBlocks<T, S>::value))
+__global__ void __launch_bounds__(128, ExplicitMinBlocks<T>::value)
     explicit_kernel(const __grid_constant__ ExplicitArgs<M, T> a)
 {
     const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;

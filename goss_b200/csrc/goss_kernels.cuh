@@ -572,22 +572,15 @@ __global__ void __launch_bounds__(128, ExplicitMinBlocks<T>::value)
 // Newton matrices of the implicit solvers are stored packed (the model's
 // lu_nnz entries of the LU structure of I - h*alpha*J, generated with the
 // structure-aware factorisation and solve that reproduce ODE::lu_factorize and
-// ODE::forward_backward_subst, ODE.cpp:69-132): in a thread-local array, or in
-// a node's slice of component-major solver-state rows (entry k of the node at
-// base[k*ld + node]).
-struct PackedRows {
-    double* base;
-    uint64_t ld;
-    __device__ __forceinline__ double& operator[](int k) const { return base[(uint64_t)k * ld]; }
-};
-
-// ... or in a tiled region: the 32 nodes of a tile keep their entries together
+// ODE::forward_backward_subst, ODE.cpp:69-132), their entries models::F64 (a
+// double whose divisions have no branches): in a thread-local array, or in a
+// tiled region: the 32 nodes of a tile keep their entries together
 // ([tile][k][32]), so a warp's lu_nnz entries are one contiguous block of
 // 256-byte rows instead of lu_nnz rows ld apart (each 2 MiB apart at 262,144
 // nodes, whose cost depended on how the allocation happened to be mapped)
 struct PackedTile {
     double* base;
-    __device__ __forceinline__ double& operator[](int k) const { return base[(uint64_t)k * 32]; }
+    __device__ __forceinline__ models::F64& operator[](int k) const { return *as_split(base + (uint64_t)k * 32); }
 };
 
 __device__ __forceinline__ PackedTile packed_tile(double* region, uint32_t node, int nnz)
@@ -602,17 +595,38 @@ __device__ __forceinline__ double l2norm(const double* v)
 #pragma unroll
     for (int i = 0; i < n; ++i)
         s += v[i] * v[i];
-    return sqrt(s);
+    return models::f64_sqrt(s);
+}
+
+// x^(4/5) of a positive convergence rate (the Newton stopping rules' eta)
+__device__ __forceinline__ double pow_4_5(double x) { return models::f64_exp(0.8 * models::f64_log(x)); }
+
+// x^(1/4) (ESDIRK23a's step-size controller)
+__device__ __forceinline__ double root4(double x) { return models::f64_sqrt(models::f64_sqrt(x)); }
+
+// x^n by squaring
+__device__ __forceinline__ double pow_int(double x, int n)
+{
+    double p = 1.0, b = x;
+    for (int k = n < 0 ? -n : n; k; k >>= 1) {
+        p = (k & 1) ? p * b : p;
+        b = b * b;
+    }
+    return n < 0 ? models::f64_div(1.0, p) : p;
 }
 
 // FP64 model right-hand side of the implicit solvers: the split form (every
 // distinct exp and reciprocal once, common factors pulled out), whose values
 // differ from the reference's operation order by rounding only; Newton
-// iterates to the same states (the implicit parity tests hold at 1e-10), and
-// the FD Jacobian, ~19 evaluations per Newton iteration, gets ~2x cheaper.
-#ifndef GOSS_IMPLICIT_SPLIT
-#define GOSS_IMPLICIT_SPLIT 1
-#endif
+// iterates to the same states (the implicit parity tests hold at 1e-10).  The
+// right-hand side, the Jacobians, the packed LU and the step control run on
+// models::F64: without the slow-path branches of CUDA's division, exp, log,
+// sqrt and pow, and with one reciprocal per pivot and per forward-difference
+// step, a 0.1 ms interval of 262,144 TT04 nodes takes (blocks of 256, 255
+// registers; at 128 or 168 registers 1.2-1.8x longer):
+//   ThetaSolver 0.89 -> 0.62 ms, + Jacobian 0.43 -> 0.27, ImplicitEuler
+//   1.47 -> 0.87, + Jacobian 0.95 -> 0.68, ESDIRK23a 3.8 -> 2.5, + Jacobian
+//   3.4 -> 2.25 (intervals of a relaxing population, min_dt 1e-4).
 // Inlined at every call site: on TT04 with the analytic Jacobian, called
 // (__noinline__) versions of these two measured 1.3x slower, and capping the
 // kernels at 128 or 170 registers (3 or 4 blocks of 128 per SM) 1.3-1.4x
@@ -620,16 +634,7 @@ __device__ __forceinline__ double l2norm(const double* v)
 template <class M>
 __device__ __forceinline__ void rhs64(const double* y, double t, const double* P, const double* F, double* out)
 {
-    if constexpr (GOSS_IMPLICIT_SPLIT)
-        M::template rhs_split<double>(y, t, P, P, F, out);
-    else
-        M::template rhs<double>(y, t, P, P, F, out);
-}
-
-template <class M, class A>
-__device__ __forceinline__ void jacobian64(const double* y, double t, const double* P, const double* F, A J)
-{
-    M::template jacobian<double>(y, t, P, P, F, J);
+    model_rhs<M, double>(y, t, P, P, F, out);
 }
 
 // The analytic Jacobian evaluated in FP32 at the FP64 point (y, t) and stored
@@ -650,53 +655,6 @@ __device__ __forceinline__ void jacobian32(const double* y, double t, const floa
     for (int k = 0; k < Dims<M>::nfp; ++k)
         Ff[k] = float(F[k]);
     M::template jacobian<float>(yf, t, P32, PD, Ff, J);
-}
-
-// ODE::compute_jacobian (ODE.cpp:47-67) into the packed Newton matrix J:
-// the model's analytic Jacobian when it was generated with one (the
-// reference's generated override), else forward differences: column i is
-// (f(y + delta_i e_i) - f(y)) / delta_i with delta_i = sqrt(1e-15 max(1e-5, |y_i|)),
-// f1 = f(y, t) supplied by the caller (the reference evaluates it first with
-// the same arguments), stored at the column's structural rows (the other
-// rows are exactly 0 in the reference too).  The perturbed state is built by
-// selects over compile-time indices, so y stays in registers (the reference
-// perturbs y[i] in place and restores it: the same values).  With the split
-// right-hand side, the generated fd_jacobian evaluates it once at y and, for
-// each column i, recomputes only the statements of the column's structural
-// rows that depend on state i (the others keep the values a full
-// re-evaluation would give).  Measured on B200 (TT04, 262,144 nodes, 0.1 ms
-// intervals): ThetaSolver 4.43 ms per interval with n full evaluations, 3.61
-// with the rows of each column's structure, 1.62 with the cones; ESDIRK23a
-// 258 -> 219 ms.
-template <class M, class A>
-__device__ __forceinline__ void compute_jacobian(const double* y, double t, const double* P, const double* F, A J,
-                                                 const double* f1)
-{
-    constexpr int n = M::num_states;
-    if constexpr (M::has_jacobian) {
-        (void)f1;
-        jacobian64<M>(y, t, P, F, J);
-    } else if constexpr (GOSS_IMPLICIT_SPLIT) {
-        M::fd_clear(J);
-        M::template fd_jacobian<double>(y, t, P, P, F, f1, J);
-    } else {
-        M::fd_clear(J);
-#pragma unroll 1
-        for (int i = 0; i < n; ++i) {
-            double ysafe = 0.0;
-#pragma unroll
-            for (int k = 0; k < n; ++k)
-                ysafe = (k == i) ? y[k] : ysafe;
-            const double max = 1e-5 > fabs(ysafe) ? 1e-5 : fabs(ysafe);
-            const double delta = sqrt(1e-15 * max);
-            double yp[n], f2[n];
-#pragma unroll
-            for (int k = 0; k < n; ++k)
-                yp[k] = (k == i) ? ysafe + delta : y[k];
-            rhs64<M>(yp, t, P, F, f2);
-            M::fd_column(i, f1, f2, delta, J);
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -763,19 +721,19 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
     // (through rhs_jacobian_sel instead: 0.69 ms, the Jacobian's statements no
     // longer interleave with f's; with forward differences through
     // rhs2_fd_jacobian: 1.5 % slower, not used).
-    constexpr bool one_eval = GOSS_THETA_ONE_EVAL && GOSS_IMPLICIT_SPLIT && !J32 && IE;
-    constexpr bool one_jac = GOSS_THETA_ONE_EVAL && GOSS_IMPLICIT_SPLIT && !J32 && !IE && M::has_jacobian;
+    constexpr bool one_eval = GOSS_THETA_ONE_EVAL && !J32 && IE;
+    constexpr bool one_jac = GOSS_THETA_ONE_EVAL && !J32 && !IE && M::has_jacobian;
     // ImplicitEuler with the FP32 Jacobian: one FP64 right-hand-side call
     // site for every iteration, the FP32 Jacobian when refactorising (1.22 ->
     // 0.77 ms per interval; for ThetaSolver, with f(y, t) of a step's first
     // iteration from the same call site, 0.57 -> 0.73 ms, not used)
-    constexpr bool one_eval32 = GOSS_THETA_ONE_EVAL && GOSS_IMPLICIT_SPLIT && J32 && IE;
+    constexpr bool one_eval32 = GOSS_THETA_ONE_EVAL && J32 && IE;
     const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = node < a.N;
     const uint32_t src = active ? node : a.N - 1;  // threads past the end only take part in the barriers
     const goss_solver_params& sp = a.sp;
     double y[n], z1[n], prev[n], yz[n], f1[n], b[n];
-    double J[M::lu_nnz];
+    models::F64 J[M::lu_nnz];
     for (int i = 0; i < n; ++i)
         y[i] = a.states[i * a.ld + src];
     double F[Dims<M>::nfp];
@@ -834,7 +792,7 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
             // refactorise, its f(y, tn) evaluation writes f(y, t) as well
             prev_pending = false;
             if (!IE && fabs(sp.theta - 1.0) > kGossEps) {
-                if (one_eval32 || (GOSS_IMPLICIT_SPLIT && !(relative_residual < sp.relative_tolerance) &&
+                if (one_eval32 || (!(relative_residual < sp.relative_tolerance) &&
                                    (recompute || always))) {
                     prev_pending = true;
                 } else {
@@ -853,7 +811,6 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
         // before f(yz) is evaluated), f(yz) and the Jacobian come from one
         // evaluation: the unperturbed statements of the forward differences,
         // or the statements the analytic Jacobian shares with f
-        constexpr bool fused = GOSS_IMPLICIT_SPLIT;
         if constexpr (one_eval32) {
             const bool want_jac = !(relative_residual < sp.relative_tolerance) && (recompute || always);
             // at a step's first iteration (yz = y) f(y, t) for the explicit part, then f(yz, tn)
@@ -876,10 +833,10 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
             // f(yz, tn), and the Jacobian when this iteration refactorises
             const bool want_jac = !(relative_residual < sp.relative_tolerance) && (recompute || always);
             if constexpr (M::has_jacobian)
-                M::template rhs_jacobian_sel<double>(yz, tn, a.P, a.P, F, t, false, want_jac, b, f1, J);
+                M::template rhs_jacobian_sel<models::F64>(as_split(yz), tn, as_split(a.P), a.P, as_split(F), t, false, want_jac, as_split(b), as_split(f1), J);
             else
-                M::template rhs_fd_jacobian_sel<double>(yz, tn, a.P, a.P, F, want_jac, f1, J);
-        } else if (fused && !(relative_residual < sp.relative_tolerance) && (recompute || always)) {
+                M::template rhs_fd_jacobian_sel<models::F64>(as_split(yz), tn, as_split(a.P), a.P, as_split(F), want_jac, as_split(f1), J);
+        } else if (!(relative_residual < sp.relative_tolerance) && (recompute || always)) {
             if constexpr (J32) {
                 // FP64 right-hand sides, the FP32 Jacobian
                 if (!IE && prev_pending) {
@@ -894,10 +851,10 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
                 // f(yz, t) into b: at the first iteration of the step (yz = y)
                 // the explicit part
                 if constexpr (M::has_jacobian) {
-                    M::template rhs2_jacobian<double>(yz, tn, a.P, a.P, F, t, b, f1, J);
+                    M::template rhs2_jacobian<models::F64>(as_split(yz), tn, as_split(a.P), a.P, as_split(F), t, as_split(b), as_split(f1), J);
                 } else {
                     M::fd_clear(J);
-                    M::template rhs2_fd_jacobian<double>(yz, tn, a.P, a.P, F, t, b, f1, J);
+                    M::template rhs2_fd_jacobian<models::F64>(as_split(yz), tn, as_split(a.P), a.P, as_split(F), t, as_split(b), as_split(f1), J);
                 }
                 if (prev_pending) {
                     for (int i = 0; i < n; ++i)
@@ -905,10 +862,10 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
                     prev_pending = false;
                 }
             } else if constexpr (M::has_jacobian) {
-                M::template rhs_jacobian<double>(yz, tn, a.P, a.P, F, f1, J);
+                M::template rhs_jacobian<models::F64>(as_split(yz), tn, as_split(a.P), a.P, as_split(F), as_split(f1), J);
             } else {
                 M::fd_clear(J);
-                M::template rhs_fd_jacobian<double>(yz, tn, a.P, a.P, F, f1, J);
+                M::template rhs_fd_jacobian<models::F64>(as_split(yz), tn, as_split(a.P), a.P, as_split(F), as_split(f1), J);
             }
         } else {
             rhs64<M>(yz, tn, a.P, F, f1);
@@ -920,8 +877,6 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
             newton_done = true;
         } else {
             if (recompute || always) {
-                if constexpr (!fused)
-                    compute_jacobian<M>(yz, tn, a.P, F, J, f1);
                 M::lu_shift(J, -ldt * alpha);
                 M::lu_factorize(J);
                 jac_comp += 1;
@@ -931,9 +886,9 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
             if (newton_iterations == 0) {
                 initial_residual = residual;
                 eta = eta > kGossEps ? eta : kGossEps;
-                eta = pow(eta, 0.8);
+                eta = pow_4_5(eta);
             } else {
-                relative_previous_residual = residual / previous_residual;
+                relative_previous_residual = models::f64_div(residual, previous_residual);
                 recompute = relative_previous_residual >= sp.max_relative_previous_residual;
                 if (relative_previous_residual >= 1) {
                     step_ok = false;
@@ -942,10 +897,10 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
                     newton_done = true;
                 } else {
                     const double scaled = std_max(
-                        pow(relative_previous_residual, (double)(sp.max_iterations - newton_iterations)), kGossEps);
-                    if (residual > (sp.kappa * sp.relative_tolerance * (1 - relative_previous_residual) / scaled))
+                        pow_int(relative_previous_residual, sp.max_iterations - newton_iterations), kGossEps);
+                    if (residual > models::f64_div(sp.kappa * sp.relative_tolerance * (1 - relative_previous_residual), scaled))
                         recompute = 1;
-                    eta = relative_previous_residual / (1.0 - relative_previous_residual);
+                    eta = models::f64_div(relative_previous_residual, 1.0 - relative_previous_residual);
                 }
             }
             if (!newton_done && newton_iterations > sp.max_iterations) {
@@ -957,7 +912,7 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
             if (!newton_done) {
                 for (int i = 0; i < n; ++i)
                     z1[i] += b[i];
-                relative_residual = residual / initial_residual;
+                relative_residual = models::f64_div(residual, initial_residual);
                 previous_residual = residual;
                 newton_iterations++;
                 newton_done = !(eta * relative_residual >= sp.kappa * sp.relative_tolerance);
@@ -1146,7 +1101,7 @@ __global__ void __launch_bounds__(GOSS_ESDIRK_THREADS, GOSS_ESDIRK_MIN_BLOCKS)
     uint8_t status = 0;
     uint64_t guard = 0;
     // ESDIRK23a::forward (ESDIRK23a.cpp:280-316)
-    double h = std_max(c.s_fac * prev_dt * pow((c.tol / loc_error), 0.25), min_dt);
+    double h = std_max(c.s_fac * prev_dt * root4(models::f64_div(c.tol, loc_error)), min_dt);
     h = std_min(h, interval);
     if (first_step) {
         prev_dt = h;
@@ -1167,7 +1122,7 @@ __global__ void __launch_bounds__(GOSS_ESDIRK_THREADS, GOSS_ESDIRK_MIN_BLOCKS)
             jac_pending += 1;
             t_jac = t0 + local_t;
         }
-        if (fabs((h - prev_dt) / prev_dt) > 0.2 || new_jacobian || jac_pending)
+        if (fabs(models::f64_div(h - prev_dt, prev_dt)) > 0.2 || new_jacobian || jac_pending)
             fact_pending = true;
         t_step = t0 + local_t;
         advance_guard = 0;
@@ -1181,7 +1136,7 @@ __global__ void __launch_bounds__(GOSS_ESDIRK_THREADS, GOSS_ESDIRK_MIN_BLOCKS)
         newton_iterations = 0;
         dz_norm = 0.0;
         newton_guard = 0;
-        eta = pow(std_max(eta, c.etamin), 0.8);
+        eta = pow_4_5(std_max(eta, c.etamin));
         phase = PH_NEWTON;
     };
     // the end of advance_one_step and of the while loop's body
@@ -1189,7 +1144,7 @@ __global__ void __launch_bounds__(GOSS_ESDIRK_THREADS, GOSS_ESDIRK_MIN_BLOCKS)
         new_jacobian = 0;
         prev_dt = h;
         local_t += h;
-        h = std_max(c.s_fac * prev_dt * pow((c.tol / loc_error), 0.25), min_dt);
+        h = std_max(c.s_fac * prev_dt * root4(models::f64_div(c.tol, loc_error)), min_dt);
         return outer_begin();
     };
     // do_step returned false: advance_one_step's retry loop
@@ -1237,14 +1192,11 @@ __global__ void __launch_bounds__(GOSS_ESDIRK_THREADS, GOSS_ESDIRK_MIN_BLOCKS)
             if constexpr (J32) {
                 (void)g1;
                 jacobian32<M>(y, t_jac, a.P32, a.P, F, jac);
-            } else if constexpr (M::has_jacobian && GOSS_IMPLICIT_SPLIT) {
-                M::template rhs_jacobian<double>(y, t_jac, a.P, a.P, F, g1, jac);
-            } else if constexpr (GOSS_IMPLICIT_SPLIT) {
-                M::fd_clear(jac);
-                M::template rhs_fd_jacobian<double>(y, t_jac, a.P, a.P, F, g1, jac);
+            } else if constexpr (M::has_jacobian) {
+                M::template rhs_jacobian<models::F64>(as_split(y), t_jac, as_split(a.P), a.P, as_split(F), as_split(g1), jac);
             } else {
-                rhs64<M>(y, t_jac, a.P, F, g1);
-                compute_jacobian<M>(y, t_jac, a.P, F, jac, g1);
+                M::fd_clear(jac);
+                M::template rhs_fd_jacobian<models::F64>(as_split(y), t_jac, as_split(a.P), a.P, as_split(F), as_split(g1), jac);
             }
             jac_comp += jac_pending;
             jac_pending = 0;
@@ -1307,12 +1259,12 @@ __global__ void __launch_bounds__(GOSS_ESDIRK_THREADS, GOSS_ESDIRK_MIN_BLOCKS)
             dz_norm = l2norm<n>(dz);
             bool fail = false;
             if (newton_iterations >= 1) {
-                const double theta = dz_norm / prev_dz_norm;
+                const double theta = models::f64_div(dz_norm, prev_dz_norm);
                 if (!(theta <= 1)) {
                     rejects += 1;
                     fail = true;
                 } else {
-                    eta = theta / (1.0 - theta);
+                    eta = models::f64_div(theta, 1.0 - theta);
                 }
             }
             if (!fail && (newton_iterations > sp.max_iterations || ++newton_guard > 100000)) {

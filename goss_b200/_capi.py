@@ -173,6 +173,8 @@ _PROTOS = {
     "goss_system_status": (C.c_int, [_sys, _u32p, C.c_int32]),
     "goss_system_node_status": (C.c_int, [_sys, C.POINTER(C.c_uint8)]),
     "goss_system_counters": (C.c_int, [_sys, _i64p, _i64p, _i64p]),
+    "goss_system_counter_totals": (C.c_int, [_sys, _i64p]),
+    "goss_system_forward_totals": (C.c_int, [_sys, C.c_double, C.c_double, _i64p]),
     "goss_system_device_states": (C.c_int, [_sys, C.POINTER(_dp), C.POINTER(C.c_uint64)]),
     "goss_system_device_field_params": (C.c_int, [_sys, C.POINTER(_dp), C.POINTER(C.c_uint64)]),
     "goss_system_set_stream": (C.c_int, [_sys, C.c_void_p]),

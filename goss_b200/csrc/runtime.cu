@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -104,6 +105,53 @@ __global__ void fill_rows_kernel(double* __restrict__ dst, uint64_t ld, uint32_t
     }
 }
 
+// A system's status in device memory: the flag word the solver kernels set,
+// and the totals of the implicit solvers' counters.
+struct StatusBlock {
+    uint32_t flags;
+    uint32_t ticket;                // blocks that have added their part
+    unsigned long long totals[3];   // Jacobians, rejected, accepted: the last sum
+    unsigned long long partial[3];  // being added up
+};
+
+// Sum of three consecutive counter rows (whole numbers held as doubles) over
+// the nodes into st->totals.  The counts are exact integers, so the order of
+// the additions does not matter.  Bound by reading the rows once (24 bytes per
+// node, in L2 after the solver kernel); copying the rows to the host and adding
+// them there took 1.6 of the 2.8 ms of a ThetaSolver interval on 262,144 nodes.
+__global__ void counter_totals_kernel(const double* __restrict__ rows, uint64_t ld, uint32_t N, StatusBlock* st)
+{
+    unsigned long long c[3] = {0, 0, 0};
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+            c[r] += (unsigned long long)(long long)rows[r * ld + i];
+    __shared__ unsigned long long s[3][8];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        for (int d = 16; d; d >>= 1)
+            c[r] += __shfl_down_sync(0xffffffffu, c[r], d);
+        if ((threadIdx.x & 31) == 0)
+            s[r][threadIdx.x >> 5] = c[r];
+    }
+    __syncthreads();
+    if (threadIdx.x)
+        return;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        for (unsigned w = 1; w < blockDim.x / 32; ++w)
+            c[r] += s[r][w];
+        atomicAdd(&st->partial[r], c[r]);
+    }
+    __threadfence();
+    if (atomicAdd(&st->ticket, 1u) == gridDim.x - 1) {  // the last block publishes and resets
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+            st->totals[r] = atomicExch(&st->partial[r], 0ull);
+        st->ticket = 0;
+    }
+}
+
 unsigned grid_for(uint64_t total, unsigned block = 256)
 {
     uint64_t g = (total + block - 1) / block;
@@ -125,9 +173,10 @@ struct goss_system {
     double* d_fparams = nullptr;
     double* d_sstate = nullptr;
     uint32_t sstate_rows = 0;
-    uint32_t* d_flags = nullptr;
+    StatusBlock* d_status = nullptr;
+    uint32_t* d_flags = nullptr;  // &d_status->flags
     uint8_t* d_node_status = nullptr;
-    double* d_stage = nullptr;  // staging for host transfers, max(n, nfp, 1) * ld doubles
+    double* d_stage = nullptr;  // staging for host transfers
     uint64_t stage_elems = 0;
     double* d_small = nullptr;  // row constants
     uint32_t* d_rows = nullptr; // row maps (field state indices / components)
@@ -216,11 +265,32 @@ int init_solver_state(goss_system* s)
     return 0;
 }
 
-int check_flags(goss_system* s)
+// first of the three counter rows of the solver state, 0 for explicit solvers
+uint32_t counter_row(const goss_system* s)
 {
-    uint32_t f = 0;
-    CUDA_TRY(s, cudaMemcpyAsync(&f, s->d_flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
+    if (s->solver == GOSS_THETA || s->solver == GOSS_IMPLICIT_EULER)
+        return 4;  // TH_JACCOMP, TH_REJECTS, TH_ACCEPTED
+    return s->solver == GOSS_ESDIRK23A ? 6 : 0;  // ES_JACCOMP, ES_REJECTS, ES_ACCEPTED
+}
+
+// Wait for the stream and raise on a node failure; with totals, sum the
+// counters on the device and read them in the same copy.
+int check_flags(goss_system* s, int64_t* totals = nullptr)
+{
+    StatusBlock b{};
+    const uint32_t row = totals ? counter_row(s) : 0;
+    if (row) {
+        const unsigned grid = std::max(1u, std::min((s->N + 255) / 256, 148u * 4));
+        counter_totals_kernel<<<grid, 256, 0, s->stream>>>(s->d_sstate + row * s->ld, s->ld, s->N, s->d_status);
+        CUDA_TRY(s, cudaGetLastError());
+    }
+    CUDA_TRY(s, cudaMemcpyAsync(&b, s->d_status, row ? offsetof(StatusBlock, partial) : sizeof(uint32_t),
+                                cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(s, cudaStreamSynchronize(s->stream));
+    if (totals)
+        for (int r = 0; r < 3; ++r)
+            totals[r] = (int64_t)b.totals[r];
+    const uint32_t f = b.flags;
     const uint32_t fresh = f & ~s->host_flags;
     s->host_flags |= f;
     if (fresh & GOSS_FLAG_NEWTON_FAILED) {
@@ -535,11 +605,13 @@ GOSS_API int goss_system_create(const goss_model_desc* m, int32_t solver, const 
         CREATE_TRY(cudaMalloc(&s->d_fparams, sizeof(double) * s->nfp * s->ld));
     if (s->sstate_rows)
         CREATE_TRY(cudaMalloc(&s->d_sstate, sizeof(double) * s->sstate_rows * s->ld));
-    CREATE_TRY(cudaMalloc(&s->d_flags, sizeof(uint32_t)));
-    CREATE_TRY(cudaMemsetAsync(s->d_flags, 0, sizeof(uint32_t), s->stream));
+    CREATE_TRY(cudaMalloc(&s->d_status, sizeof(StatusBlock)));
+    s->d_flags = &s->d_status->flags;
+    CREATE_TRY(cudaMemsetAsync(s->d_status, 0, sizeof(StatusBlock), s->stream));
     CREATE_TRY(cudaMalloc(&s->d_node_status, s->ld));
     CREATE_TRY(cudaMemsetAsync(s->d_node_status, 0, s->ld, s->stream));
-    s->stage_elems = (uint64_t)std::max<uint32_t>(std::max(s->n, s->nfp), 1) * s->ld;
+    // host transfers: states, field parameters, the three counter rows
+    s->stage_elems = (uint64_t)std::max<uint32_t>(std::max(s->n, s->nfp), s->sstate_rows ? 3 : 1) * s->ld;
     CREATE_TRY(cudaMalloc(&s->d_stage, sizeof(double) * s->stage_elems));
     CREATE_TRY(cudaMalloc(&s->d_small, sizeof(double) * std::max<uint32_t>(std::max(s->n, s->nfp), 64)));
 #undef CREATE_TRY
@@ -564,7 +636,7 @@ GOSS_API int goss_system_destroy(goss_system* s)
     cudaFree(s->d_states);
     cudaFree(s->d_fparams);
     cudaFree(s->d_sstate);
-    cudaFree(s->d_flags);
+    cudaFree(s->d_status);
     cudaFree(s->d_node_status);
     cudaFree(s->d_stage);
     cudaFree(s->d_small);
@@ -947,6 +1019,26 @@ GOSS_API int goss_system_forward(goss_system* s, double t, double interval)
     return rc;
 }
 
+GOSS_API int goss_system_forward_totals(goss_system* s, double t, double interval, int64_t* totals)
+{
+    if (!s || !totals)
+        return fail(s ? &s->last_error : nullptr, GOSS_ERR_ARGUMENT, "NULL argument");
+    int rc = set_device(s);
+    if (!rc)
+        rc = launch_forward(s, t, interval);
+    if (!rc)
+        rc = check_flags(s, totals);
+    return rc;
+}
+
+GOSS_API int goss_system_counter_totals(goss_system* s, int64_t* totals)
+{
+    if (!s || !totals)
+        return fail(s ? &s->last_error : nullptr, GOSS_ERR_ARGUMENT, "NULL argument");
+    int rc = set_device(s);
+    return rc ? rc : check_flags(s, totals);
+}
+
 GOSS_API int goss_system_forward_async(goss_system* s, double t, double interval)
 {
     if (!s)
@@ -1208,12 +1300,9 @@ GOSS_API int goss_system_counters(const goss_system* cs, int64_t* jac_comp, int6
     auto* s = const_cast<goss_system*>(cs);
     if (!s)
         return fail(nullptr, GOSS_ERR_ARGUMENT, "NULL system");
-    uint32_t rows[3];
-    if (s->solver == GOSS_THETA || s->solver == GOSS_IMPLICIT_EULER) {
-        rows[0] = 4, rows[1] = 5, rows[2] = 6;  // TH_JACCOMP, TH_REJECTS, TH_ACCEPTED
-    } else if (s->solver == GOSS_ESDIRK23A) {
-        rows[0] = 6, rows[1] = 7, rows[2] = 8;  // ES_JACCOMP, ES_REJECTS, ES_ACCEPTED
-    } else {
+    const uint32_t row = counter_row(s);
+    const uint32_t rows[3] = {row, row + 1, row + 2};
+    if (!row) {
         for (uint32_t i = 0; i < s->N; ++i) {
             if (jac_comp)
                 jac_comp[i] = 0;

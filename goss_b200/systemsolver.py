@@ -91,15 +91,11 @@ class ODESystemSolver:
         for i, v in enumerate(self._ode._params):
             _capi.check(self._L.goss_system_set_parameter(self._h, i, float(v)), self._h)
 
-    def _update_counters(self) -> None:
-        if isinstance(self._solver, ImplicitODESolver):
-            jc, rj, ac = self.counters()
-            self._solver._counters["jac_comp"] = int(jc.sum())
-            self._solver._counters["rejected"] = int(rj.sum())
-            self._solver._counters["accepted"] = int(ac.sum())
-            if isinstance(self._solver, ESDIRK):
-                self._solver._counters["ndtsa"] = int(ac.sum())
-                self._solver._counters["ndtsr"] = int(rj.sum())
+    def _set_counters(self, totals) -> None:
+        c = self._solver._counters
+        c["jac_comp"], c["rejected"], c["accepted"] = totals
+        if isinstance(self._solver, ESDIRK):
+            c["ndtsa"], c["ndtsr"] = c["accepted"], c["rejected"]
 
     # -- reference API ---------------------------------------------------------
     @property
@@ -215,8 +211,12 @@ class ODESystemSolver:
 
     def forward(self, t: float, interval: float) -> None:
         self._sync_params()
-        _capi.check(self._L.goss_system_forward(self._h, float(t), float(interval)), self._h)
-        self._update_counters()
+        if isinstance(self._solver, ImplicitODESolver):
+            totals = (C.c_int64 * 3)()
+            _capi.check(self._L.goss_system_forward_totals(self._h, float(t), float(interval), totals), self._h)
+            self._set_counters(totals)
+        else:
+            _capi.check(self._L.goss_system_forward(self._h, float(t), float(interval)), self._h)
 
     def solve(self, t: np.ndarray) -> np.ndarray:
         """Field states at every time of ``t``: shape (len(t), num_nodes, num_field_states)."""
@@ -228,7 +228,10 @@ class ODESystemSolver:
         self._sync_params()
         _capi.check(self._L.goss_system_solve(self._h, _capi.ptr(field_states), _capi.ptr(t), num_steps,
                                               int(self._tangled_storage)), self._h)
-        self._update_counters()
+        if isinstance(self._solver, ImplicitODESolver):
+            totals = (C.c_int64 * 3)()
+            _capi.check(self._L.goss_system_counter_totals(self._h, totals), self._h)
+            self._set_counters(totals)
         return field_states
 
     # -- GPU extras ------------------------------------------------------------

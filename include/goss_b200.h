@@ -336,6 +336,13 @@ GOSS_API int goss_system_node_status(const goss_system* sys, uint8_t* out);
 /* Counters of the implicit solvers per node: jacobian computations,
  * rejected steps, accepted steps (any pointer may be NULL). */
 GOSS_API int goss_system_counters(const goss_system* sys, int64_t* jac_comp, int64_t* rejected, int64_t* accepted);
+/* The same counters summed over the nodes on the device: totals[3] = jacobian
+ * computations, rejected steps, accepted steps (0 for the explicit solvers).
+ * Waits for the system's stream and reports node failures as
+ * goss_system_synchronize does. */
+GOSS_API int goss_system_counter_totals(goss_system* sys, int64_t* totals);
+/* goss_system_forward, with the totals after it from the same synchronisation. */
+GOSS_API int goss_system_forward_totals(goss_system* sys, double t, double interval, int64_t* totals);
 
 /* Device-resident access for callers that keep data on the GPU. */
 GOSS_API int goss_system_device_states(goss_system* sys, double** states, uint64_t* ld);

@@ -164,6 +164,7 @@ _PROTOS = {
     "goss_system_get_states": (C.c_int, [_sys, _dp]),
     "goss_system_set_states": (C.c_int, [_sys, _dp]),
     "goss_system_set_parameter": (C.c_int, [_sys, C.c_uint32, C.c_double]),
+    "goss_system_set_parameters": (C.c_int, [_sys, _dp, C.c_uint32]),
     "goss_system_get_parameter": (C.c_int, [_sys, C.c_uint32, _dp]),
     "goss_system_reset_default": (C.c_int, [_sys]),
     "goss_system_set_num_threads": (C.c_int, [_sys, C.c_uint32]),

@@ -612,6 +612,7 @@ GOSS_API int goss_system_create(const goss_model_desc* m, int32_t solver, const 
     CREATE_TRY(cudaMemsetAsync(s->d_node_status, 0, s->ld, s->stream));
     // host transfers: states, field parameters, the three counter rows
     s->stage_elems = (uint64_t)std::max<uint32_t>(std::max(s->n, s->nfp), s->sstate_rows ? 3 : 1) * s->ld;
+    s->stage_elems = std::max<uint64_t>(s->stage_elems, 16384);  // small systems: the times of a whole solve
     CREATE_TRY(cudaMalloc(&s->d_stage, sizeof(double) * s->stage_elems));
     CREATE_TRY(cudaMalloc(&s->d_small, sizeof(double) * std::max<uint32_t>(std::max(s->n, s->nfp), 64)));
 #undef CREATE_TRY
@@ -1234,6 +1235,14 @@ GOSS_API int goss_system_set_parameter(goss_system* s, uint32_t index, double va
     return 0;
 }
 
+GOSS_API int goss_system_set_parameters(goss_system* s, const double* values, uint32_t count)
+{
+    if (!s || count != s->m->num_parameters || (count && !values))
+        return fail(s ? &s->last_error : nullptr, GOSS_ERR_ARGUMENT, "expected every model parameter");
+    std::copy(values, values + count, s->params.begin());
+    return 0;
+}
+
 GOSS_API int goss_system_get_parameter(const goss_system* s, uint32_t index, double* value)
 {
     if (!s || !value || index >= s->m->num_parameters)
@@ -1362,12 +1371,22 @@ GOSS_API int goss_system_solve(goss_system* s, double* field_states, const doubl
         return 0;
     uint64_t chunk = per ? std::max<uint64_t>(1, (256ull << 20) / (8 * per)) : 1;
     chunk = std::min<uint64_t>(chunk, nt - 1);
+    // the staging buffer when it holds all times or at least 32 of them (small
+    // systems: an allocation takes longer than their whole solve)
     double* d_out = nullptr;
+    double* d_own = nullptr;
     if (per) {
-        CUDA_TRY(s, cudaMalloc(&d_out, sizeof(double) * per * chunk));
+        const uint64_t staged = s->stage_elems / per;
+        if (staged >= std::min<uint64_t>(chunk, 32)) {
+            chunk = std::min(chunk, staged);
+            d_out = s->d_stage;
+        } else {
+            CUDA_TRY(s, cudaMalloc(&d_own, sizeof(double) * per * chunk));
+            d_out = d_own;
+        }
         rc = ensure_rows(s, s->fsi.data(), nfs);
         if (rc) {
-            cudaFree(d_out);
+            cudaFree(d_own);
             return rc;
         }
     }
@@ -1404,7 +1423,7 @@ GOSS_API int goss_system_solve(goss_system* s, double* field_states, const doubl
     if (!rc && !per)
         rc = check_flags(s);
     cudaStreamSynchronize(s->stream);
-    cudaFree(d_out);
+    cudaFree(d_own);
     return rc;
 }
 

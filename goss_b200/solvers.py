@@ -12,6 +12,7 @@ BasicImplicitEuler, ESDIRK4O32) are not provided.
 from __future__ import annotations
 
 import abc
+import functools
 from enum import Enum
 from typing import Any, Dict, Optional
 
@@ -19,6 +20,13 @@ import numpy as np
 
 from . import _capi
 from .ode import ODE
+
+
+@functools.lru_cache(maxsize=None)
+def _default_c_params(kind: int) -> bytes:
+    sp = _capi.SolverParams()
+    _capi.check(_capi.lib().goss_solver_default_params(kind, sp))
+    return bytes(sp)
 
 
 class ODESolver(abc.ABC):
@@ -119,8 +127,7 @@ class ODESolver(abc.ABC):
 
     def c_params(self) -> _capi.SolverParams:
         """Parameters in the layout of ``goss_solver_params``."""
-        sp = _capi.SolverParams()
-        _capi.check(_capi.lib().goss_solver_default_params(self._kind, sp))
+        sp = _capi.SolverParams.from_buffer_copy(_default_c_params(self._kind))
         sp.ldt = float(self._ldt)
         for k, v in self._params.items():
             if hasattr(sp, k):
@@ -151,10 +158,9 @@ class ODESolver(abc.ABC):
         t = np.asarray(t, dtype=np.float64)
         y = np.zeros((t.size, self.num_states))
         y[0, :] = y0
-        cur = np.array(y0, dtype=np.float64)
-        for it in range(1, t.size):
-            self.forward(cur, t[it - 1], t[it] - t[it - 1])
-            y[it, :] = cur
+        if t.size > 1:
+            # every time enqueued at once, the states copied back together
+            self._one_node()._solve_states(y[0], t, y)
         return y
 
 

@@ -88,8 +88,8 @@ class ODESystemSolver:
     # -- parameter plumbing ---------------------------------------------------
     def _sync_params(self) -> None:
         _capi.check(self._L.goss_system_set_solver_params(self._h, self._solver.c_params()), self._h)
-        for i, v in enumerate(self._ode._params):
-            _capi.check(self._L.goss_system_set_parameter(self._h, i, float(v)), self._h)
+        p = np.ascontiguousarray(self._ode._params, dtype=np.float64)
+        _capi.check(self._L.goss_system_set_parameters(self._h, _capi.ptr(p), p.size), self._h)
 
     def _set_counters(self, totals) -> None:
         c = self._solver._counters
@@ -228,11 +228,31 @@ class ODESystemSolver:
         self._sync_params()
         _capi.check(self._L.goss_system_solve(self._h, _capi.ptr(field_states), _capi.ptr(t), num_steps,
                                               int(self._tangled_storage)), self._h)
+        self._read_counters()
+        return field_states
+
+    def _read_counters(self) -> None:
         if isinstance(self._solver, ImplicitODESolver):
             totals = (C.c_int64 * 3)()
             _capi.check(self._L.goss_system_counter_totals(self._h, totals), self._h)
             self._set_counters(totals)
-        return field_states
+
+    def _solve_states(self, states: np.ndarray, t: np.ndarray, out: np.ndarray) -> None:
+        """All states at t[1:] into out[1:] (float64, C-contiguous, (len(t),
+        num_nodes, num_states)), from ``states`` at t[0]."""
+        self._set_states(states)
+        t = np.ascontiguousarray(t, dtype=np.float64)
+        self._sync_params()
+        u32 = C.POINTER(C.c_uint32)
+        every = np.arange(self._ode.num_states, dtype=np.uint32)
+        fsi = np.array(self._ode.field_state_indices, dtype=np.uint32)
+        _capi.check(self._L.goss_system_set_field_state_indices(self._h, every.ctypes.data_as(u32), every.size),
+                    self._h)
+        try:
+            _capi.check(self._L.goss_system_solve(self._h, _capi.ptr(out), _capi.ptr(t), t.size, 1), self._h)
+        finally:
+            self._L.goss_system_set_field_state_indices(self._h, fsi.ctypes.data_as(u32), fsi.size)
+        self._read_counters()
 
     # -- GPU extras ------------------------------------------------------------
     def forward_async(self, t: float, interval: float) -> None:

@@ -314,6 +314,8 @@ GOSS_API int goss_system_set_states(goss_system* sys, const double* states);
 
 /* Uniform model parameters (ParameterizedODE::set_parameter/get_parameter by index). */
 GOSS_API int goss_system_set_parameter(goss_system* sys, uint32_t index, double value);
+/* All of them at once; count must be the model's number of parameters. */
+GOSS_API int goss_system_set_parameters(goss_system* sys, const double* values, uint32_t count);
 GOSS_API int goss_system_get_parameter(const goss_system* sys, uint32_t index, double* value);
 
 /* reset_default() (ODESystemSolver.cpp:192-216); also resets implicit solver state */

@@ -284,6 +284,46 @@ __host__ __device__ __forceinline__ double sqrt(double x)
 
 namespace goss_b200 {
 
+// Two FP32 numbers in one 64-bit register pair.  sm_100a adds, multiplies and
+// fuses both halves with one instruction, which halves the issue slots of
+// arithmetic that comes in pairs (the kernels that use it are bound by
+// instruction issue); each half rounds and flushes as the scalar instruction.
+struct F32x2 {
+    unsigned long long v;
+    F32x2() = default;
+    __device__ __forceinline__ F32x2(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+    __device__ __forceinline__ explicit F32x2(float a) : F32x2(a, a) {}
+    __device__ __forceinline__ void unpack(float& a, float& b) const
+    {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    }
+};
+__device__ __forceinline__ F32x2 operator+(F32x2 a, F32x2 b)
+{
+    F32x2 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F32x2 operator-(F32x2 a, F32x2 b)
+{
+    F32x2 r;
+    asm("sub.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F32x2 operator*(F32x2 a, F32x2 b)
+{
+    F32x2 r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F32x2 vfma(F32x2 a, F32x2 b, F32x2 c)
+{
+    F32x2 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
+
 // phi1(x) = (e^x - 1)/x with phi1(0) = 1, in single precision.
 //
 // The generalised Rush-Larsen update y + b/a (e^{a h} - 1) equals
@@ -293,22 +333,20 @@ namespace goss_b200 {
 // digits), so the FP32 kernels use phi1 instead: for |x| < 1/4 the Taylor
 // series sum_k x^k/(k+1)! truncated after x^6 (relative truncation error
 // < (1/4)^7/8! < 2e-9), otherwise (e^x - 1)/x with the SFU exponential.
-__device__ __forceinline__ float phi1f(float x)
+template <typename V>
+__device__ __forceinline__ V phi1f_small(V x)
 {
-    const float ax = fabsf(x);
-    if (ax < 0.25f) {
-        // Horner form of 1 + x/2 + x^2/6 + x^3/24 + x^4/120 + x^5/720 + x^6/5040
-        float p = 1.0f / 5040.0f;
-        p = fmaf(p, x, 1.0f / 720.0f);
-        p = fmaf(p, x, 1.0f / 120.0f);
-        p = fmaf(p, x, 1.0f / 24.0f);
-        p = fmaf(p, x, 1.0f / 6.0f);
-        p = fmaf(p, x, 0.5f);
-        p = fmaf(p, x, 1.0f);
-        return p;
-    }
-    return __fdividef(__expf(x) - 1.0f, x);
+    // Horner form of 1 + x/2 + x^2/6 + x^3/24 + x^4/120 + x^5/720 + x^6/5040
+    V p = V(1.0f / 5040.0f);
+    p = vfma(p, x, V(1.0f / 720.0f));
+    p = vfma(p, x, V(1.0f / 120.0f));
+    p = vfma(p, x, V(1.0f / 24.0f));
+    p = vfma(p, x, V(1.0f / 6.0f));
+    p = vfma(p, x, V(0.5f));
+    return vfma(p, x, V(1.0f));
 }
+__device__ __forceinline__ float phi1f_large(float x) { return __fdividef(__expf(x) - 1.0f, x); }
+__device__ __forceinline__ float phi1f(float x) { return fabsf(x) < 0.25f ? phi1f_small(x) : phi1f_large(x); }
 
 }  // namespace goss_b200
 

@@ -102,3 +102,31 @@ def test_exponential_increment():
     quant = np.abs(np.asarray(f, float)) * np.where(np.abs(a) > 1e-8, rounding, 1e-8)
     tol = 4 * np.minimum(quant, np.abs(ref) + 2) + 2e-15 * (np.abs(ref) + 2)
     assert np.all(np.abs(got - ref) <= tol)
+
+
+@pytest.mark.parametrize("states", [1, 2, 21, 22])  # no pair, one pair, a full group and an odd state, two groups
+@pytest.mark.parametrize("solver", ["GRL1", "GRL2"])
+def test_single_precision_increment(states, solver):
+    """x_i' = a_i x_i + 0.3 in single precision, a_i from 1e-4 to 40 per step on
+    both sides of the polynomial's range, the states side by side in pairs."""
+    a = -np.logspace(-4, np.log10(40.0), states) if states > 1 else np.array([-0.2])
+    a = np.where(np.arange(states) % 3 == 2, np.minimum(-a, 3.0), a)
+    text = f"states({', '.join(f'x{i}=2.0' for i in range(states))})\n"
+    text += "".join(f"dx{i}_dt = {float(a[i])!r}*x{i} + 0.3\n" for i in range(states))
+    ode = goss.ParameterizedODE(parse_ode_text(text, f"split_single_{states}"))
+    s = goss.solvers.solver_mapper[solver](ode)
+    s.internal_time_step = 1.0
+    system = goss.ODESystemSolver(33, s, ode, precision="single")
+    system.forward(0.0, 1.0)
+    f = 2 * a + 0.3
+    if solver == "GRL2":
+        f = a * (2 + f * np.expm1(a / 2) / a) + 0.3
+    ref = 2 + f * np.expm1(a) / a
+    # right-hand side and product in FP32 (6e-8 each of |a x| + 0.3), phi1 at
+    # worst the cancellation of e^x - 1 next to |x| = 1/4 (1.2e-7 / 0.22); GRL2
+    # carries the half step's error through a
+    scale = (np.abs(a) * np.maximum(2, np.abs(ref)) + 0.3) * np.expm1(a) / a
+    tol = 3e-6 * scale * (1 + (np.abs(a) if solver == "GRL2" else 0)) + 1e-12
+    got = system.states
+    assert np.all(got == got[0])  # every node of a warp and of the ragged block
+    assert np.all(np.abs(got[0] - ref) <= tol)

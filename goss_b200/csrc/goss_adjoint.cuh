@@ -41,10 +41,13 @@
 // (ten Tusscher-Panfilov, 65,536 nodes x 2,000 steps, backward pass):
 //   FP32: blocks of up to 128 threads, 2 per SM (255 registers), lockstep
 //         28.0 ms; 256 x 1: 29.3 ms; register caps of 168 or 128 (3 or 4
-//         blocks of 128) spill more than the extra warps gain: 37.5 ms; with
-//         the record's tape (65,536 nodes x 40,000 steps, 368 of 400
-//         segments taped) 2, 3, 4 blocks: 445, 650, 716 ms;
+//         blocks of 128) spill more than the extra warps gain: 37.5 ms (with
+//         the record's tape 2.0-2.3x the time);
 //   FP64: 256 x 1: 207 ms; 128 x 2: 215 ms.
+// Since then (65,536 nodes x 1,000 steps, taped): FP32 10.87 -> 9.64 ms with
+// the step's seeds (phi1 and its derivative of every state) in packed FP32
+// under one branch; FP64, 200 steps, 17.1 -> 10.1 ms with the sweeps on
+// models::F64, whose division, exp and log have no branches.
 // (the shape of the backward follows the arithmetic of its VJPs)
 template <typename T>
 struct AdjointShape {
@@ -57,67 +60,135 @@ struct AdjointShape {
 
 namespace goss_b200 {
 
-// phi1(x) = (e^x - 1)/x and phi1'(x) = (e^x (x - 1) + 1)/x^2 in FP64:
-// Taylor series sum_k x^k/(k+1)! and sum_k (k+1) x^k/(k+2)! for |x| < 0.1
-// (truncation below 1e-17 relative), closed forms otherwise.
-__device__ __forceinline__ double phi1d(double x)
+// phi1(x) = (e^x - 1)/x and phi1'(x) = (e^x (x - 1) + 1)/x^2.  FP64, |x| < 1/8:
+// f64_phi1_small and the Taylor series sum_k (k+1) x^k/(k+2)! to x^9
+// (truncation 4e-17 relative), even and odd terms apart; closed forms beyond.
+__device__ __forceinline__ double dphi1d_small(double x)
 {
-    if (fabs(x) < 0.1) {
-        double p = 1.0 / 362880.0;
-        p = fma(p, x, 1.0 / 40320.0);
-        p = fma(p, x, 1.0 / 5040.0);
-        p = fma(p, x, 1.0 / 720.0);
-        p = fma(p, x, 1.0 / 120.0);
-        p = fma(p, x, 1.0 / 24.0);
-        p = fma(p, x, 1.0 / 6.0);
-        p = fma(p, x, 0.5);
-        p = fma(p, x, 1.0);
-        return p;
-    }
-    return expm1(x) / x;
+    const double g = x * x;
+    double a = 9.0 / 3628800.0, b = 10.0 / 39916800.0;
+    a = fma(a, g, 7.0 / 40320.0);
+    b = fma(b, g, 8.0 / 362880.0);
+    a = fma(a, g, 5.0 / 720.0);
+    b = fma(b, g, 6.0 / 5040.0);
+    a = fma(a, g, 3.0 / 24.0);
+    b = fma(b, g, 4.0 / 120.0);
+    a = fma(a, g, 0.5);
+    b = fma(b, g, 2.0 / 6.0);
+    return fma(b, x, a);
 }
 
-__device__ __forceinline__ double dphi1d(double x)
+// FP32: Taylor series to x^7 for |x| < 1/4 (truncation < 2e-9), closed forms otherwise
+template <typename V>
+__device__ __forceinline__ V dphi1f_small(V x)
 {
-    if (fabs(x) < 0.1) {
-        // sum_{k=0}^{9} (k+1) x^k / (k+2)!
-        double p = 10.0 / 39916800.0;
-        p = fma(p, x, 9.0 / 3628800.0);
-        p = fma(p, x, 8.0 / 362880.0);
-        p = fma(p, x, 7.0 / 40320.0);
-        p = fma(p, x, 6.0 / 5040.0);
-        p = fma(p, x, 5.0 / 720.0);
-        p = fma(p, x, 4.0 / 120.0);
-        p = fma(p, x, 3.0 / 24.0);
-        p = fma(p, x, 2.0 / 6.0);
-        p = fma(p, x, 0.5);
-        return p;
-    }
-    return (exp(x) * (x - 1.0) + 1.0) / (x * x);
+    // sum_{k=0}^{7} (k+1) x^k / (k+2)!
+    V p = V(8.0f / 362880.0f);
+    p = vfma(p, x, V(7.0f / 40320.0f));
+    p = vfma(p, x, V(6.0f / 5040.0f));
+    p = vfma(p, x, V(5.0f / 720.0f));
+    p = vfma(p, x, V(4.0f / 120.0f));
+    p = vfma(p, x, V(3.0f / 24.0f));
+    p = vfma(p, x, V(2.0f / 6.0f));
+    return vfma(p, x, V(0.5f));
 }
-
-// FP32: Taylor series to x^6 for |x| < 1/4 (truncation < 2e-9), closed forms otherwise
-__device__ __forceinline__ float dphi1f(float x)
+__device__ __forceinline__ float dphi1f_large(float x)
 {
-    if (fabsf(x) < 0.25f) {
-        // sum_{k=0}^{7} (k+1) x^k / (k+2)!
-        float p = 8.0f / 362880.0f;
-        p = fmaf(p, x, 7.0f / 40320.0f);
-        p = fmaf(p, x, 6.0f / 5040.0f);
-        p = fmaf(p, x, 5.0f / 720.0f);
-        p = fmaf(p, x, 4.0f / 120.0f);
-        p = fmaf(p, x, 3.0f / 24.0f);
-        p = fmaf(p, x, 2.0f / 6.0f);
-        p = fmaf(p, x, 0.5f);
-        return p;
-    }
     return __fdividef(__expf(x) * (x - 1.0f) + 1.0f, x * x);
 }
 
-__device__ __forceinline__ double phi1t(double x) { return phi1d(x); }
-__device__ __forceinline__ float phi1t(float x) { return phi1f(x); }
-__device__ __forceinline__ double dphi1t(double x) { return dphi1d(x); }
-__device__ __forceinline__ float dphi1t(float x) { return dphi1f(x); }
+// Cotangents of the linear coefficients and right-hand sides of one GRL1 step:
+// bbar_i = lambda_i h phi1(a_i h), abar_i = lambda_i b_i h^2 phi1'(a_i h).
+// FP64 in groups of four states under one branch (as grl_increments).
+template <int N>
+__device__ __forceinline__ void grl1_seed_group(const double* lv, const double* lin, const double* rhs, double h,
+                                                double* abar, double* bbar)
+{
+    double x[N], p[N], d[N];
+    int far = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        x[i] = lin[i] * h;
+        p[i] = models::f64_phi1_small(x[i]);
+        d[i] = dphi1d_small(x[i]);
+        far = max(far, __double2hiint(x[i]) & 0x7fffffff);
+    }
+    if (far >= 0x3fc00000) {  // |x| >= 1/8, infinite or NaN
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            if ((__double2hiint(x[i]) & 0x7fffffff) >= 0x3fc00000) {
+                const double e = models::f64_exp(x[i]), r = models::f64_rcp(x[i]);
+                p[i] = (e - 1.0) * r;
+                d[i] = (e * (x[i] - 1.0) + 1.0) * (r * r);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        bbar[i] = lv[i] * h * p[i];
+        abar[i] = lv[i] * rhs[i] * h * h * d[i];
+    }
+}
+
+template <int n>
+__device__ __forceinline__ void grl1_seed(const double* lv, const double* lin, const double* rhs, double h,
+                                          double* abar, double* bbar)
+{
+    constexpr int rest = n % 4;
+#pragma unroll
+    for (int i = 0; i + 4 <= n; i += 4)
+        grl1_seed_group<4>(lv + i, lin + i, rhs + i, h, abar + i, bbar + i);
+    if constexpr (rest != 0)
+        grl1_seed_group<rest>(lv + n - rest, lin + n - rest, rhs + n - rest, h, abar + n - rest, bbar + n - rest);
+}
+
+// FP32: two states at a time in packed arithmetic, all under one branch; the
+// operations of the scalar form in its order.
+template <int n>
+__device__ __forceinline__ void grl1_seed(const float* lv, const float* lin, const float* rhs, float h, float* abar,
+                                          float* bbar)
+{
+    constexpr int pairs = n / 2, P = pairs > 0 ? pairs : 1;
+    const F32x2 hh(h);
+    F32x2 p[P], d[P];
+    float far[P], all = 0.0f;
+#pragma unroll
+    for (int i = 0; i < pairs; ++i) {
+        const F32x2 x = F32x2(lin[2 * i], lin[2 * i + 1]) * hh;
+        float x0, x1;
+        x.unpack(x0, x1);
+        p[i] = phi1f_small(x);
+        d[i] = dphi1f_small(x);
+        far[i] = fmaxf(fabsf(x0), fabsf(x1));
+        all = fmaxf(all, far[i]);
+    }
+    if (all >= 0.25f) {
+#pragma unroll
+        for (int i = 0; i < pairs; ++i) {
+            if (far[i] >= 0.25f) {
+                const float x0 = lin[2 * i] * h, x1 = lin[2 * i + 1] * h;
+                float p0, p1, d0, d1;
+                p[i].unpack(p0, p1);
+                d[i].unpack(d0, d1);
+                const bool n0 = fabsf(x0) < 0.25f, n1 = fabsf(x1) < 0.25f;
+                p[i] = F32x2(n0 ? p0 : phi1f_large(x0), n1 ? p1 : phi1f_large(x1));
+                d[i] = F32x2(n0 ? d0 : dphi1f_large(x0), n1 ? d1 : dphi1f_large(x1));
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < pairs; ++i) {
+        const F32x2 l(lv[2 * i], lv[2 * i + 1]);
+        (l * hh * p[i]).unpack(bbar[2 * i], bbar[2 * i + 1]);
+        (l * F32x2(rhs[2 * i], rhs[2 * i + 1]) * hh * hh * d[i]).unpack(abar[2 * i], abar[2 * i + 1]);
+    }
+    if constexpr (n % 2 != 0) {
+        const float x = lin[n - 1] * h;
+        const bool near = fabsf(x) < 0.25f;
+        bbar[n - 1] = lv[n - 1] * h * (near ? phi1f_small(x) : phi1f_large(x));
+        abar[n - 1] = lv[n - 1] * rhs[n - 1] * h * h * (near ? dphi1f_small(x) : dphi1f_large(x));
+    }
+}
 
 template <class M, typename T>
 struct AdjointArgs {
@@ -234,19 +305,17 @@ __device__ __forceinline__ void reverse_step_grl1(const T* yt, double lt, double
 {
     constexpr int n = M::num_states;
     constexpr int nfp = Dims<M>::nfp;
+    using V = split_t<T>;
     const T h = T(ldt);
     T lv[n], ybar[n], Fbar[nfp];
     for (int i = 0; i < n; ++i)
         lv[i] = lam[i].value();
-    auto seed = [&](const T* lin, const T* rhs, T* abar, T* bbar) {
-#pragma unroll
-        for (int i = 0; i < n; ++i) {
-            const T x = lin[i] * h;
-            bbar[i] = lv[i] * h * phi1t(x);
-            abar[i] = lv[i] * rhs[i] * h * h * dphi1t(x);
-        }
+    auto seed = [&](const V* lin, const V* rhs, V* abar, V* bbar) {
+        grl1_seed<n>(lv, reinterpret_cast<const T*>(lin), reinterpret_cast<const T*>(rhs), h,
+                     reinterpret_cast<T*>(abar), reinterpret_cast<T*>(bbar));
     };
-    M::template linearized_vjp<T>(yt, lt, P, PD, F, seed, ybar, Fbar);
+    M::template linearized_vjp<V>(as_split(yt), lt, as_split(P), PD, as_split(F), seed, as_split(ybar),
+                                  as_split(Fbar));
     for (int i = 0; i < n; ++i)
         lam[i].add(ybar[i]);
     for (int q = 0; q < M::num_field_params; ++q)
@@ -279,7 +348,7 @@ __device__ __forceinline__ void reverse_step_rk4(const T* yt, double lt, double 
         }
     }
     T lv[n], kb[n], ysum[n];
-    const T w6 = h / T(6.0), w3 = h / T(3.0);
+    const T w6 = T(split_t<T>(h) / split_t<T>(6.0)), w3 = T(split_t<T>(h) / split_t<T>(3.0));
     for (int i = 0; i < n; ++i) {
         lv[i] = lam[i].value();
         kb[i] = w6 * lv[i];
@@ -292,12 +361,13 @@ __device__ __forceinline__ void reverse_step_rk4(const T* yt, double lt, double 
         for (int i = 0; i < n; ++i)
             u[i] = st == 0 ? yt[i] : yt[i] + c * (st == 3 ? k3[i] : st == 2 ? k2[i] : k1[i]);
         T ub[n], Fb[nfp];
-        auto seed = [&](const T*, T* bbar) {
+        auto seed = [&](const split_t<T>*, split_t<T>* bbar) {
 #pragma unroll
             for (int i = 0; i < n; ++i)
-                bbar[i] = kb[i];
+                bbar[i] = split_t<T>(kb[i]);
         };
-        M::template rhs_vjp<T>(u, ts, P, PD, F, seed, ub, Fb);
+        M::template rhs_vjp<split_t<T>>(as_split(u), ts, as_split(P), PD, as_split(F), seed, as_split(ub),
+                                        as_split(Fb));
         const T w = st == 1 ? w6 : w3;
         for (int i = 0; i < n; ++i) {
             ysum[i] = ysum[i] + ub[i];
@@ -416,7 +486,10 @@ adjoint_kernel(const __grid_constant__ AdjointArgs<M, T> a)
 // the multiple of 32 (<= AdjointShape<T>::block) minimising that product (ties:
 // the larger block) -- e.g. for 65,536 nodes on 148 SMs with two blocks per
 // SM: 112 threads (two nearly full waves) instead of 128 (a second wave on
-// 108 of 148 SMs).
+// 108 of 148 SMs).  A grid below one wave counts the blocks it puts on an SM,
+// not those that would fit: 2,001 nodes in FP64 take blocks of 32 (one warp on
+// each of 63 SMs) instead of 256 (eight on each of 8): GRL1 100 steps 1.80 ->
+// 1.13 ms, 8,000 nodes (blocks of 64) 1.87 -> 1.19 ms.
 template <class M, typename T, Explicit S, typename R = T>
 inline unsigned adjoint_block(uint32_t num_nodes, size_t shm)
 {
@@ -434,7 +507,7 @@ inline unsigned adjoint_block(uint32_t num_nodes, size_t shm)
         const uint64_t grid = (num_nodes + b - 1) / b;
         const uint64_t slots = (uint64_t)active * sms;
         const uint64_t waves = (grid + slots - 1) / slots;
-        const uint64_t cost = waves * (uint64_t)active * b;
+        const uint64_t cost = (waves > 1 ? waves * (uint64_t)active : (grid + sms - 1) / sms) * b;
         if (cost < best_cost) {
             best_cost = cost;
             best = b;

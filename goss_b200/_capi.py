@@ -152,6 +152,8 @@ _PROTOS = {
     "goss_system_get_solver_params": (C.c_int, [_sys, C.POINTER(SolverParams)]),
     "goss_system_forward": (C.c_int, [_sys, C.c_double, C.c_double]),
     "goss_system_forward_async": (C.c_int, [_sys, C.c_double, C.c_double]),
+    "goss_system_exchange_field_states": (C.c_int, [_sys, C.c_void_p, C.c_void_p, C.c_int32]),
+    "goss_system_step_field_states": (C.c_int, [_sys, C.c_double, C.c_double, C.c_void_p, C.c_void_p]),
     "goss_system_synchronize": (C.c_int, [_sys]),
     "goss_system_solve": (C.c_int, [_sys, _dp, _dp, C.c_uint64, C.c_int32]),
     "goss_system_set_field_state_indices": (C.c_int, [_sys, _u32p, C.c_uint32]),

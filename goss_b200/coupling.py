@@ -24,6 +24,7 @@ from typing import Dict, Mapping, Optional, Tuple
 
 import numpy as np
 
+from . import _capi
 from .systemsolver import ODESystemSolver
 
 
@@ -118,12 +119,38 @@ class FieldStateCoupling:
                              f"{'' if self.num_fields == 1 else ' ' + str(self.num_fields)})")
         return v if v.dim() == 2 else v.view(-1, 1)
 
+    def _plain(self, v) -> bool:
+        """Whether the exchange kernels can take ``v``'s memory as it is: a
+        plain contiguous tensor of this device outside autograd (reverse and
+        forward mode), at most 64 fields.  Anything else goes through torch's
+        own indexing."""
+        import torch
+        from torch.autograd import forward_ad
+
+        return (type(v) is torch.Tensor and v.is_contiguous() and v.device == self.device and not v.requires_grad
+                and not v.is_neg() and self.num_fields <= 64 and forward_ad._current_level < 0
+                and all(d.dtype == torch.int64 and d.is_contiguous() and d.numel() == self.systems[lab].num_nodes
+                        for lab, d in self.dofs.items()))
+
+    def _touched(self, *tensors) -> None:
+        """Tell autograd that the kernels wrote into these tensors."""
+        from torch.autograd.graph import increment_version
+
+        for t in tensors:
+            increment_version(t)
+
     def to_field_states(self, v) -> None:
         """Copy the PDE vector into the populations' field states
         (``DOLFINODESystemSolver.to_field_states``)."""
         import torch
 
         v2 = self._vector(v)
+        if self._plain(v):
+            for lab, s in self.systems.items():
+                _capi.check(s._L.goss_system_exchange_field_states(s._h, v.data_ptr(), self.dofs[lab].data_ptr(), 0),
+                            s._h)
+                self._touched(*self._views[lab])
+            return
         with torch.cuda.stream(self.stream):
             for lab, views in self._views.items():
                 vals = v2.index_select(0, self.dofs[lab])
@@ -136,6 +163,12 @@ class FieldStateCoupling:
         import torch
 
         v2 = self._vector(v)
+        if self._plain(v):
+            for lab, s in self.systems.items():
+                _capi.check(s._L.goss_system_exchange_field_states(s._h, v.data_ptr(), self.dofs[lab].data_ptr(), 1),
+                            s._h)
+            self._touched(v)
+            return
         with torch.cuda.stream(self.stream):
             for lab, views in self._views.items():
                 vals = torch.stack(views, dim=1)
@@ -152,6 +185,15 @@ class FieldStateCoupling:
         of every population, from_field_states (``DOLFINODESystemSolver.step``),
         all enqueued on the coupling's stream without waiting."""
         t0, t1 = interval
+        self._vector(v)
+        if self._plain(v):
+            # population by population: their dofs are disjoint
+            for lab, s in self.systems.items():
+                _capi.check(s._L.goss_system_step_field_states(s._h, float(t0), float(t1) - float(t0), v.data_ptr(),
+                                                               self.dofs[lab].data_ptr()), s._h)
+                self._touched(*self._views[lab])
+            self._touched(v)
+            return
         self.to_field_states(v)
         for s in self.systems.values():
             s.forward_async(float(t0), float(t1) - float(t0))

@@ -93,6 +93,31 @@ __global__ void gather_kernel(double* __restrict__ dst, const double* __restrict
     }
 }
 
+// Field states exchanged with a vector indexed by dof: row k of the map holds
+// field k, vec[dofs[node]*count + k] <-> states[row[k]*ld + node].  One launch
+// for all fields of a population, the row map in the argument block (no copy,
+// no allocation, so it can be captured).  Bound by its launch at the sizes of a
+// mesh partition: 8 + 16 bytes per node and field.
+constexpr uint32_t kMaxFields = 64;
+struct FieldRows {
+    uint32_t count;
+    uint32_t row[kMaxFields];
+};
+__global__ void exchange_kernel(double* __restrict__ states, uint64_t ld, uint32_t N, double* __restrict__ vec,
+                                const int64_t* __restrict__ dofs, const __grid_constant__ FieldRows f, int to_vector)
+{
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+        double* const v = vec + (uint64_t)dofs[i] * f.count;
+        for (uint32_t k = 0; k < f.count; ++k) {
+            double* const s = states + (uint64_t)f.row[k] * ld + i;
+            if (to_vector)
+                v[k] = *s;
+            else
+                *s = v[k];
+        }
+    }
+}
+
 // dst[r*ld + node] = values[r] for every node < N (rows 0..k-1)
 __global__ void fill_rows_kernel(double* __restrict__ dst, uint64_t ld, uint32_t N, uint32_t k,
                                  const double* __restrict__ values)
@@ -1116,7 +1141,43 @@ int to_host(goss_system* s, double* host, const double* src, uint32_t k, const u
     return 0;
 }
 
+// enqueue one direction of an exchange with a device vector
+int exchange(goss_system* s, double* vec, const int64_t* dofs, int to_vector)
+{
+    FieldRows f{};
+    f.count = (uint32_t)s->fsi.size();
+    if (!f.count || !s->N)
+        return 0;
+    if (f.count > kMaxFields)
+        return fail(&s->last_error, GOSS_ERR_ARGUMENT, "more than %u field states", kMaxFields);
+    std::copy(s->fsi.begin(), s->fsi.end(), f.row);
+    exchange_kernel<<<grid_for(s->N), 256, 0, s->stream>>>(s->d_states, s->ld, s->N, vec, dofs, f, to_vector);
+    CUDA_TRY(s, cudaGetLastError());
+    return 0;
+}
+
 }  // namespace
+
+GOSS_API int goss_system_exchange_field_states(goss_system* s, double* vector, const int64_t* dofs, int32_t to_vector)
+{
+    if (!s || !vector || !dofs)
+        return fail(s ? &s->last_error : nullptr, GOSS_ERR_ARGUMENT, "NULL argument");
+    int rc = set_device(s);
+    return rc ? rc : exchange(s, vector, dofs, to_vector);
+}
+
+GOSS_API int goss_system_step_field_states(goss_system* s, double t, double interval, double* vector,
+                                           const int64_t* dofs)
+{
+    if (!s || !vector || !dofs)
+        return fail(s ? &s->last_error : nullptr, GOSS_ERR_ARGUMENT, "NULL argument");
+    int rc = set_device(s);
+    if (!rc)
+        rc = exchange(s, vector, dofs, 0);
+    if (!rc)
+        rc = launch_forward(s, t, interval);
+    return rc ? rc : exchange(s, vector, dofs, 1);
+}
 
 GOSS_API int goss_system_set_field_state_indices(goss_system* s, const uint32_t* idx, uint32_t count)
 {

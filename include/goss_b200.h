@@ -351,6 +351,18 @@ GOSS_API int goss_system_device_states(goss_system* sys, double** states, uint64
 GOSS_API int goss_system_device_field_params(goss_system* sys, double** field_params, uint64_t* ld);
 GOSS_API int goss_system_set_stream(goss_system* sys, void* stream);
 GOSS_API int goss_system_forward_async(goss_system* sys, double t, double interval);
+/* Field states exchanged with a device vector of num_field_states values per
+ * dof, vector[dofs[node]*num_field_states + k], dofs[num_nodes] on the device
+ * (distinct, not checked here), enqueued on the system's stream without
+ * waiting: into the field states (to_vector 0) or into the vector (1); at most
+ * 64 field states. */
+GOSS_API int goss_system_exchange_field_states(goss_system* sys, double* vector, const int64_t* dofs,
+                                               int32_t to_vector);
+/* One step of an operator splitting (DOLFINODESystemSolver::step,
+ * python/goss/dolfinutils.py:740-780): field states from the vector, forward,
+ * field states to the vector, all enqueued. */
+GOSS_API int goss_system_step_field_states(goss_system* sys, double t, double interval, double* vector,
+                                           const int64_t* dofs);
 GOSS_API int goss_system_synchronize(goss_system* sys);
 
 /* Batched model evaluation on host arrays: states [count][n], times [count],

@@ -304,6 +304,13 @@ __device__ __forceinline__ F32x2 operator+(F32x2 a, F32x2 b)
     asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
     return r;
 }
+// rounded toward zero
+__device__ __forceinline__ F32x2 vadd_rz(F32x2 a, F32x2 b)
+{
+    F32x2 r;
+    asm("add.rz.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
 __device__ __forceinline__ F32x2 operator-(F32x2 a, F32x2 b)
 {
     F32x2 r;

@@ -679,12 +679,11 @@ __device__ __forceinline__ void explicit_node_from(const NodeIO& a, uint32_t nod
 }
 
 // Resident blocks of 128 threads per SM the explicit kernels are compiled for
-// (register cap 65536 / (128 * blocks)).  FP64: 3 (168 registers): measured on
-// B200 (TP06, 262,144 nodes x 100 steps, four fields), blocks 2 / 3 / 4: GRL1
-// 3.91 / 3.73 / 3.96 ms, GRL2 8.23 / 8.24 / 9.26, RK4 12.4 / 12.2 / 12.9; more
-// warps hide the FP64 latencies better than the spills cost up to there.
-// FP32: uncapped (150 registers for TP06 GRL1, 3 blocks per SM); capping it at
-// 128 registers measured 2.77e10 against 2.91e10 cell-steps/s.
+// (register cap 65536 / (128 * blocks)).  FP32: uncapped (150 registers for
+// TP06 GRL1, 3 blocks per SM; capped at 128 it measured 1-13 % slower at every
+// size).  FP64: 3 (168 registers), whose extra warps hide the FP64 latencies
+// better than the spills cost; GRL1, GRL2 and RK4 also 2 (255 registers), which
+// is faster while the grid leaves an SM no third block, see explicit_blocks.
 #ifndef GOSS_EXPLICIT_MIN_BLOCKS_FP32
 #define GOSS_EXPLICIT_MIN_BLOCKS_FP32 1
 #endif
@@ -692,10 +691,33 @@ template <typename T>
 struct ExplicitMinBlocks {
     static constexpr int value = sizeof(T) == 4 ? GOSS_EXPLICIT_MIN_BLOCKS_FP32 : 3;
 };
+template <typename T, Explicit S>
+constexpr bool explicit_two_shapes =
+    sizeof(T) == 8 && (S == Explicit::GRL1 || S == Explicit::GRL2 || S == Explicit::RK4);
 
-template <class M, typename T, Explicit S>
-__global__ void __launch_bounds__(128, ExplicitMinBlocks<T>::value)
-    explicit_kernel(const __grid_constant__ ExplicitArgs<M, T> a)
+// Resident blocks per SM to run `grid` FP64 blocks of 128 with: the time of the
+// full waves and of the last one under either register cap.  Time of a wave
+// with one, two (three) blocks on every SM, measured for TP06 GRL1, 100 steps:
+// 0.455, 0.604 ms at 255 registers, 0.484, 0.620, 0.848 ms at 168 (RK4 1.41,
+// 1.84 against 1.82, 2.13; GRL2 0.94, 1.24 against 1.12, 1.34).  E.g. one node
+// 2, 50,021 nodes 3 (0.85 against 1.12 ms), 65,536 nodes 2 (1.16 against
+// 1.34 ms), 262,144 nodes 3 (3.75 against 4.04 ms).
+inline int explicit_blocks(unsigned grid)
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+        return 3;
+    auto time = [&](unsigned k, const double* wave) {
+        const unsigned slots = k * (unsigned)sms, full = grid / slots, rest = grid % slots;
+        return full * wave[k] + wave[(rest + sms - 1) / sms];
+    };
+    constexpr double wide[] = {0.0, 0.455, 0.604}, narrow[] = {0.0, 0.484, 0.620, 0.848};
+    return time(2, wide) < time(3, narrow) ? 2 : 3;
+}
+
+template <class M, typename T, Explicit S, int Blocks>
+__global__ void __launch_bounds__(128, Blocks) explicit_kernel(const __grid_constant__ ExplicitArgs<M, T> a)
 {
     const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
     if (node >= a.N)
@@ -1567,7 +1589,14 @@ inline int launch_explicit(const goss_launch* L)
     const unsigned grid = (L->num_nodes + block - 1) / block;
     if (grid == 0)
         return 0;
-    explicit_kernel<M, T, S><<<grid, block, 0, (cudaStream_t)L->stream>>>(a);
+    const cudaStream_t st = (cudaStream_t)L->stream;
+    if constexpr (explicit_two_shapes<T, S>) {
+        if (block == 128 && explicit_blocks(grid) == 2) {
+            explicit_kernel<M, T, S, 2><<<grid, block, 0, st>>>(a);
+            return cudaPeekAtLastError() == cudaSuccess ? 0 : GOSS_ERR_CUDA;
+        }
+    }
+    explicit_kernel<M, T, S, ExplicitMinBlocks<T>::value><<<grid, block, 0, st>>>(a);
     return cudaPeekAtLastError() == cudaSuccess ? 0 : GOSS_ERR_CUDA;
 }
 

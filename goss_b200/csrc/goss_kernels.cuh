@@ -858,36 +858,32 @@ enum ThetaRows { TH_ETA = 0, TH_RECOMPUTE, TH_ALWAYS, TH_JUSTREFINED, TH_JACCOMP
 #ifndef GOSS_THETA_MIN_BLOCKS
 #define GOSS_THETA_MIN_BLOCKS 1
 #endif
-#ifndef GOSS_THETA_ONE_EVAL
-#define GOSS_THETA_ONE_EVAL 1
-#endif
 template <class M, bool IE, bool J32 = false>
 __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
     theta_kernel(const __grid_constant__ ImplicitArgs<M> a)
 {
     constexpr int n = M::num_states;
-    // One inlined copy of the model evaluation where that is faster (an
-    // instruction-cache effect: the per-node code is far larger than the
-    // cache).  ImplicitEuler, which keeps its Jacobian and mostly evaluates
-    // f alone: every iteration through rhs_jacobian_sel or rhs_fd_jacobian_sel
-    // (the Jacobian's own statements under a run-time condition).
-    // ThetaSolver with the analytic Jacobian, which refactorises in (nearly)
-    // every iteration: every refactorising iteration through rhs2_jacobian,
-    // f(y, t) used at a step's first iteration only (the time-dependent
-    // statements are evaluated at t each time).  Measured (TT04, 262,144
-    // nodes, 0.1 ms intervals, A/B in one process): ImplicitEuler 1.30 -> 1.04
-    // ms per interval with the analytic Jacobian, 1.88 -> 1.54 ms with forward
-    // differences; ThetaSolver with the analytic Jacobian 0.61 -> 0.55 ms
-    // (through rhs_jacobian_sel instead: 0.69 ms, the Jacobian's statements no
-    // longer interleave with f's; with forward differences through
-    // rhs2_fd_jacobian: 1.5 % slower, not used).
-    constexpr bool one_eval = GOSS_THETA_ONE_EVAL && !J32 && IE;
-    constexpr bool one_jac = GOSS_THETA_ONE_EVAL && !J32 && !IE && M::has_jacobian;
+    // One inlined copy of the model evaluation (an instruction-cache effect:
+    // the per-node code is far larger than the cache, and instruction fetch is
+    // the top stall).  ImplicitEuler, which keeps its Jacobian and mostly
+    // evaluates f alone: every iteration through rhs_jacobian_sel or
+    // rhs_fd_jacobian_sel (the Jacobian's own statements under a run-time
+    // condition).  ThetaSolver, which refactorises in (nearly) every
+    // iteration: every refactorising iteration through rhs2_jacobian or
+    // rhs2_fd_jacobian, f(y, t) used at a step's first iteration only (the
+    // time-dependent statements are evaluated at t each time).  Measured when
+    // introduced (TT04, 262,144 nodes, 0.1 ms intervals, A/B in one process):
+    // ImplicitEuler 1.30 -> 1.04 ms per interval with the analytic Jacobian,
+    // 1.88 -> 1.54 ms with forward differences; ThetaSolver with the analytic
+    // Jacobian 0.61 -> 0.55 ms (through rhs_jacobian_sel instead: 0.69 ms, the
+    // Jacobian's statements no longer interleave with f's), with forward
+    // differences 0.578 -> 0.559 ms.
+    constexpr bool one_eval = !J32 && IE;
     // ImplicitEuler with the FP32 Jacobian: one FP64 right-hand-side call
     // site for every iteration, the FP32 Jacobian when refactorising (1.22 ->
     // 0.77 ms per interval; for ThetaSolver, with f(y, t) of a step's first
     // iteration from the same call site, 0.57 -> 0.73 ms, not used)
-    constexpr bool one_eval32 = GOSS_THETA_ONE_EVAL && J32 && IE;
+    constexpr bool one_eval32 = J32 && IE;
     const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = node < a.N;
     const uint32_t src = active ? node : a.N - 1;  // threads past the end only take part in the barriers
@@ -1010,9 +1006,9 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
                 }
                 rhs64<M>(yz, tn, a.P, F, f1);
                 jacobian32<M>(yz, tn, a.P32, a.P, F, J);
-            } else if (!IE && (one_jac || prev_pending)) {
-                // f(yz, t) into b: at the first iteration of the step (yz = y)
-                // the explicit part
+            } else {
+                // ThetaSolver: f(yz, t) into b, at the first iteration of the
+                // step (yz = y) the explicit part
                 if constexpr (M::has_jacobian) {
                     M::template rhs2_jacobian<models::F64>(as_split(yz), tn, PS, a.P, as_split(F), t, as_split(b),
                                                            as_split(f1), J);
@@ -1026,11 +1022,6 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
                         prev[i] = (1 - sp.theta) * b[i];
                     prev_pending = false;
                 }
-            } else if constexpr (M::has_jacobian) {
-                M::template rhs_jacobian<models::F64>(as_split(yz), tn, PS, a.P, as_split(F), as_split(f1), J);
-            } else {
-                M::fd_clear(J);
-                M::template rhs_fd_jacobian<models::F64>(as_split(yz), tn, PS, a.P, as_split(F), as_split(f1), J);
             }
         } else {
             rhs64<M>(yz, tn, a.P, F, f1);

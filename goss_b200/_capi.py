@@ -12,7 +12,7 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 RUNTIME_SO = PKG / "_lib" / "libgoss_b200.so"
 
-ABI_VERSION = 4
+ABI_VERSION = 5
 
 (GOSS_EXPLICIT_EULER, GOSS_RK4, GOSS_GRL1, GOSS_GRL2, GOSS_THETA, GOSS_ESDIRK23A, GOSS_RL1, GOSS_RL2, GOSS_RK2,
  GOSS_IMPLICIT_EULER) = range(10)

@@ -328,9 +328,23 @@ int check_flags(goss_system* s, int64_t* totals = nullptr)
     return 0;
 }
 
-int launch_forward(goss_system* s, double t, double interval)
+// Whether the solver's kernels take a schedule, outputs and an exchange vector
+// (explicit_extended in goss_kernels.cuh) and can map the field states, which
+// have to be distinct rows.
+bool takes_schedule(const goss_system* s)
 {
-    goss_launch L{};
+    if (s->fsi.empty() || s->precision == GOSS_FP64_PRINTED ||
+        !(s->solver == GOSS_EXPLICIT_EULER || s->solver == GOSS_RK4 || s->solver == GOSS_GRL1 ||
+          s->solver == GOSS_GRL2))
+        return false;
+    std::vector<uint32_t> r(s->fsi);
+    std::sort(r.begin(), r.end());
+    return r.size() <= 127 && std::adjacent_find(r.begin(), r.end()) == r.end();
+}
+
+int launch_forward(goss_system* s, double t, double interval, const goss_launch& extra = goss_launch{})
+{
+    goss_launch L = extra;
     L.solver = s->solver;
     L.precision = s->precision;
     L.num_nodes = s->N;
@@ -1172,8 +1186,18 @@ GOSS_API int goss_system_step_field_states(goss_system* s, double t, double inte
     if (!s || !vector || !dofs)
         return fail(s ? &s->last_error : nullptr, GOSS_ERR_ARGUMENT, "NULL argument");
     int rc = set_device(s);
-    if (!rc)
-        rc = exchange(s, vector, dofs, 0);
+    if (rc)
+        return rc;
+    if (takes_schedule(s)) {
+        // gather, forward and scatter in the solver's own launch
+        goss_launch L{};
+        L.field_rows = s->fsi.data();
+        L.num_fields = (uint32_t)s->fsi.size();
+        L.vector = vector;
+        L.dofs = dofs;
+        return launch_forward(s, t, interval, L);
+    }
+    rc = exchange(s, vector, dofs, 0);
     if (!rc)
         rc = launch_forward(s, t, interval);
     return rc ? rc : exchange(s, vector, dofs, 1);
@@ -1416,6 +1440,62 @@ GOSS_API int goss_system_device_field_params(goss_system* s, double** fp, uint64
     return 0;
 }
 
+namespace {
+
+// goss_system_solve with an explicit solver: all output times that fit the
+// chunk buffer in one launch, the kernel writing the field states after each
+// (a launch and a gather per time took 8 us of a small system's solve each).
+// The buffer holds the schedule, then the outputs: the staging buffer when that
+// takes all times or 32 of them, else one of up to 256 MB.
+int solve_scheduled(goss_system* s, double* field_states, const double* t, uint64_t nt, int32_t tangled)
+{
+    const uint64_t per = (uint64_t)s->N * s->fsi.size(), times = nt - 1;
+    const uint64_t head = sizeof(goss_forward) / sizeof(double);
+    uint64_t chunk = std::min<uint64_t>(times, std::max<uint64_t>(1, (256ull << 20) / (8 * per)));
+    double* d_own = nullptr;
+    double* d_buf = s->d_stage;
+    const uint64_t staged = s->stage_elems / (per + head);
+    if (staged >= std::min<uint64_t>(chunk, 32)) {
+        chunk = std::min(chunk, staged);
+    } else {
+        CUDA_TRY(s, cudaMalloc(&d_own, sizeof(double) * (per + head) * chunk));
+        d_buf = d_own;
+    }
+    int rc = 0;
+    std::vector<goss_forward> schedule(chunk);
+    for (uint64_t first = 0; first < times && !rc; first += chunk) {
+        const uint64_t count = std::min(chunk, times - first);
+        for (uint64_t k = 0; k < count; ++k) {
+            const double dt = t[first + k + 1] - t[first + k];
+            const uint64_t nsteps = s->sp.ldt > 0 ? (unsigned long)ceil(dt / s->sp.ldt - 1.0E-12) : 1ul;
+            schedule[k] = goss_forward{t[first + k], dt / nsteps, nsteps};
+        }
+        goss_launch L{};
+        L.field_rows = s->fsi.data();
+        L.num_fields = (uint32_t)s->fsi.size();
+        L.forwards = (uint32_t)count;
+        L.schedule = reinterpret_cast<const goss_forward*>(d_buf);
+        L.out = d_buf + head * chunk;
+        L.tangled = tangled;
+        cudaError_t e = cudaMemcpyAsync(d_buf, schedule.data(), sizeof(goss_forward) * count, cudaMemcpyHostToDevice,
+                                        s->stream);
+        if (e == cudaSuccess)
+            rc = launch_forward(s, t[first], t[first + 1] - t[first], L);
+        if (e == cudaSuccess && !rc)
+            e = cudaMemcpyAsync(field_states + (first + 1) * per, L.out, sizeof(double) * per * count,
+                                cudaMemcpyDeviceToHost, s->stream);
+        if (e != cudaSuccess)
+            rc = fail(&s->last_error, GOSS_ERR_CUDA, "solve: %s", cudaGetErrorString(e));
+        if (!rc)
+            rc = check_flags(s);  // synchronises the stream
+    }
+    cudaStreamSynchronize(s->stream);
+    cudaFree(d_own);
+    return rc;
+}
+
+}  // namespace
+
 // ODESystemSolver::solve (ODESystemSolver.cpp:81-99).  The field states of
 // every output time are gathered on the device into a chunk buffer and
 // copied back once per chunk.
@@ -1430,6 +1510,8 @@ GOSS_API int goss_system_solve(goss_system* s, double* field_states, const doubl
     const uint64_t per = (uint64_t)s->N * nfs;
     if (nt < 2)
         return 0;
+    if (per && takes_schedule(s))
+        return solve_scheduled(s, field_states, t, nt, tangled);
     uint64_t chunk = per ? std::max<uint64_t>(1, (256ull << 20) / (8 * per)) : 1;
     chunk = std::min<uint64_t>(chunk, nt - 1);
     // the staging buffer when it holds all times or at least 32 of them (small

@@ -35,7 +35,7 @@ extern "C" {
 #define GOSS_API
 #endif
 
-#define GOSS_B200_ABI_VERSION 4u
+#define GOSS_B200_ABI_VERSION 5u
 
 /* Solver kinds: the reference solver classes on this path. */
 enum goss_solver_kind {
@@ -99,6 +99,13 @@ typedef struct goss_solver_params {
 
 /* One kernel launch of a solver over a node range (filled by the runtime,
  * consumed by a model module's launch function). */
+/* One forward of a schedule: its start time, internal step and number of steps. */
+typedef struct goss_forward {
+    double t;
+    double ldt;
+    uint64_t nsteps;
+} goss_forward;
+
 typedef struct goss_launch {
     int32_t solver;
     int32_t precision;
@@ -116,6 +123,21 @@ typedef struct goss_launch {
     double interval;
     uint64_t max_loop;       /* guard for adaptive loops (0 = default) */
     void* stream;            /* cudaStream_t */
+    /* For ExplicitEuler, RK4, GRL1 and GRL2; all zero: one forward on t, interval.
+     * Field k of num_fields is the state row field_rows[k] (host, distinct). */
+    const uint32_t* field_rows;
+    uint32_t num_fields;
+    /* several consecutive forwards (device [forwards]) instead of t, interval,
+     * and the field states after each of them into out[forwards] (device,
+     * [num_nodes][num_fields] each when tangled, else [num_fields][num_nodes]) */
+    uint32_t forwards;
+    const goss_forward* schedule;
+    double* out;
+    int32_t tangled;
+    /* field states read from vector[dofs[node]*num_fields + k] instead of the
+     * state rows before, and written there as well as to the rows after (device) */
+    double* vector;
+    const int64_t* dofs;
 } goss_launch;
 
 /* Batched evaluation of the model on device arrays (used by ODE.eval and the

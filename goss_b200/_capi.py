@@ -117,6 +117,7 @@ class AdjointLaunch(C.Structure):
         ("tape", C.c_void_p),
         ("taped_segments", C.c_uint32),
         ("reverse_precision", C.c_int32),
+        ("keep_stages", C.c_int32),
     ]
 
 

@@ -27,6 +27,10 @@ import numpy as np
 from . import _capi
 from .ode import ParameterizedODE
 
+# most device memory the recompute's scratch takes for keeping RK4's stages (at
+# 2,001 nodes and 100 steps per segment it is 0.14 GB)
+_STAGE_SCRATCH_BYTES = 2 << 30
+
 _AdjointFn = C.CFUNCTYPE(C.c_int, C.POINTER(_capi.AdjointLaunch))
 
 
@@ -96,8 +100,13 @@ class SolverTrace:
         dev = self.device
         self._checkpoints = torch.zeros((self.num_checkpoints, rows, self.ld), dtype=cp_dtype, device=dev)
         sld = (self.N + 255) // 256 * 256 + 256
-        self._scratch = torch.zeros((self.K, self.n, sld), dtype=cp_dtype, device=dev)
-        segment_bytes = self.K * self.n * sld * self._scratch.element_size()
+        segment_bytes = self.K * self.n * sld * cp_dtype.itemsize
+        # RK4 in double precision: room for three stage derivatives of every
+        # step beside its input while that stays small
+        self._keep_stages = (solver == "RK4" and self.precision == _capi.GOSS_FP64
+                             and 4 * segment_bytes <= _STAGE_SCRATCH_BYTES)
+        self._scratch = torch.zeros((self.K, 4 * self.n if self._keep_stages else self.n, sld), dtype=cp_dtype,
+                                    device=dev)
         if tape_bytes == "auto":
             tape_bytes = torch.cuda.mem_get_info(dev)[0] - int(tape_reserve)
         elif not isinstance(tape_bytes, numbers.Integral) or isinstance(tape_bytes, bool):
@@ -139,6 +148,7 @@ class SolverTrace:
         L.trace = self._trace.data_ptr()
         L.trace_bar = trace_bar.data_ptr() if trace_bar is not None else None
         L.scratch = self._scratch.data_ptr()
+        L.keep_stages = self._keep_stages and self.taped_segments < self.num_checkpoints
         L.field_params_bar = fp_bar.data_ptr() if fp_bar is not None else None
         L.states_bar = states_bar.data_ptr() if states_bar is not None else None
         L.flags = self._flags.data_ptr()

@@ -35,11 +35,14 @@
 // Launch shape of the adjoint kernel per arithmetic type: the largest threads
 // per block (a multiple of 32, at most 256) and the minimum resident blocks
 // per SM it is compiled for (its register cap is 65536 / (threads * blocks)).
-// With GOSS_ADJOINT_LOCKSTEP the warps of a block synchronise after every step
-// of the recompute and reverse loops, so they walk the large straight-line
-// step code together and share instruction-cache lines.  Measured on B200
+// In FP64 the warps of a block synchronise after every step of the recompute and
+// reverse loops, so they walk the large straight-line step code together and
+// share instruction-cache lines (65,536 nodes x 200 GRL1 steps 7.37 -> 7.22 ms,
+// 30,000 nodes x 100 RK4 steps 9.09 -> 7.78); FP32, whose step code is a third
+// as long, is faster without (65,536 x 1,000 GRL1 steps 9.64 -> 9.37 ms).
+// Measured on B200
 // (ten Tusscher-Panfilov, 65,536 nodes x 2,000 steps, backward pass):
-//   FP32: blocks of up to 128 threads, 2 per SM (255 registers), lockstep
+//   FP32: blocks of up to 128 threads, 2 per SM (255 registers)
 //         28.0 ms; 256 x 1: 29.3 ms; register caps of 168 or 128 (3 or 4
 //         blocks of 128) spill more than the extra warps gain: 37.5 ms (with
 //         the record's tape 2.0-2.3x the time);
@@ -53,10 +56,8 @@ template <typename T>
 struct AdjointShape {
     static constexpr unsigned block = sizeof(T) == 4 ? 128 : 256;
     static constexpr unsigned min_blocks = sizeof(T) == 4 ? 2 : 1;
+    static constexpr bool lockstep = sizeof(T) == 8;
 };
-#ifndef GOSS_ADJOINT_LOCKSTEP
-#define GOSS_ADJOINT_LOCKSTEP 1
-#endif
 
 namespace goss_b200 {
 
@@ -326,16 +327,26 @@ __device__ __forceinline__ void reverse_step_grl1(const T* yt, double lt, double
 // rhs_vjp are instantiated once.  The stage inputs are formed from the step's
 // input value (in FP32 its high word; the forward adds the low word as well,
 // a difference of at most half an FP32 ulp of the state).
+// kept: the step's first three stage derivatives (rows ld apart) where the
+// recompute kept them, which saves evaluating them again here -- the same
+// values; FP64, 2,001 nodes x 200 steps 12.6 -> 10.1 ms, 30,000 x 100 9.2 -> 6.7.
 template <class M, typename T>
 __device__ __forceinline__ void reverse_step_rk4(const T* yt, double lt, double ldt, const T* P, const double* PD,
-                                                 const T* F, Acc<T>* lam, double* gF)
+                                                 const T* F, Acc<T>* lam, double* gF, const T* kept, uint64_t ld)
 {
     constexpr int n = M::num_states;
     constexpr int nfp = Dims<M>::nfp;
     const T h = T(ldt), hh = T(0.5 * ldt);
     T k1[n], k2[n], k3[n], u[n];
+    if (kept) {
+        for (int i = 0; i < n; ++i) {
+            k1[i] = kept[i * ld];
+            k2[i] = kept[(n + i) * ld];
+            k3[i] = kept[(2 * n + i) * ld];
+        }
+    }
 #pragma unroll 1
-    for (int st = 0; st < 3; ++st) {
+    for (int st = kept ? 3 : 0; st < 3; ++st) {
         const double ts = st == 0 ? lt : lt + 0.5 * ldt;
         for (int i = 0; i < n; ++i)
             u[i] = st == 0 ? yt[i] : yt[i] + hh * (st == 1 ? k1[i] : k2[i]);
@@ -383,7 +394,9 @@ __device__ __forceinline__ void reverse_step_rk4(const T* yt, double lt, double 
 // R is the arithmetic of the step VJPs and of lambda: T, or double over an
 // FP32 trajectory (the recompute keeps T, so the same trajectory is
 // differentiated; only the VJP arithmetic changes).
-template <class M, typename T, Explicit S, typename R = T>
+// Keep: the recompute keeps RK4's stage derivatives in scratch (a kernel of its
+// own: where it has none to read, the choice at run time cost 5 %).
+template <class M, typename T, Explicit S, typename R = T, bool Keep = false>
 __global__ void __launch_bounds__(AdjointShape<R>::block, AdjointShape<R>::min_blocks)
 adjoint_kernel(const __grid_constant__ AdjointArgs<M, T> a)
 {
@@ -436,7 +449,9 @@ adjoint_kernel(const __grid_constant__ AdjointArgs<M, T> a)
         // the input state of every step of the segment: from the record's
         // tape, or recomputed from the checkpoint into scratch
         const T* seg = scratch;
+        [[maybe_unused]] bool kept = Keep;
         if ((uint32_t)c >= num_cp - a.taped_segments) {
+            kept = false;
             seg = a.tape + (uint64_t)(c - (num_cp - a.taped_segments)) * K * n * a.sld + src;
         } else {
             Acc<T> y[n];
@@ -445,12 +460,19 @@ adjoint_kernel(const __grid_constant__ AdjointArgs<M, T> a)
                         ((uint64_t)c * rows + n + i) * a.ld + src, y[i]);
             for (uint32_t k = 0; k < len; ++k) {
                 for (int i = 0; i < n; ++i)
-                    scratch[((uint64_t)k * n + i) * a.sld] = y[i].value();
-                if (k + 1 < len)
+                    scratch[((uint64_t)k * (Keep ? 4 * n : n) + i) * a.sld] = y[i].value();
+                if constexpr (Keep) {
+                    // the last step's stages are needed too
+                    explicit_step<M, T, S>(y, s_time[k], ldt, a.P, a.PD, F, T(kGrlDelta), [&](int st, const T* kst) {
+                        if (st < 3)
+                            for (int i = 0; i < n; ++i)
+                                scratch[((uint64_t)k * 4 * n + (st + 1) * n + i) * a.sld] = kst[i];
+                    });
+                } else if (k + 1 < len) {
                     explicit_step<M, T, S>(y, s_time[k], ldt, a.P, a.PD, F, T(kGrlDelta));
-#if GOSS_ADJOINT_LOCKSTEP
-                __syncthreads();
-#endif
+                }
+                if constexpr (AdjointShape<R>::lockstep)
+                    __syncthreads();
             }
         }
         // reverse through the segment
@@ -461,15 +483,18 @@ adjoint_kernel(const __grid_constant__ AdjointArgs<M, T> a)
                 lam[a.trace_state].add(R(a.trace_bar[j * a.ld + src]));
             }
             R yt[n];
+            const T* const row = seg + (uint64_t)k * (Keep && kept ? 4 * n : n) * a.sld;
             for (int i = 0; i < n; ++i)
-                yt[i] = R(seg[((uint64_t)k * n + i) * a.sld]);
+                yt[i] = R(row[i * a.sld]);
             if constexpr (S == Explicit::GRL1)
                 reverse_step_grl1<M, R>(yt, s_time[k], ldt, PR, a.PD, FR, lam, gF);
+            else if constexpr (Keep)
+                reverse_step_rk4<M, R>(yt, s_time[k], ldt, PR, a.PD, FR, lam, gF, kept ? row + n * a.sld : nullptr,
+                                       a.sld);
             else
-                reverse_step_rk4<M, R>(yt, s_time[k], ldt, PR, a.PD, FR, lam, gF);
-#if GOSS_ADJOINT_LOCKSTEP
-            __syncthreads();
-#endif
+                reverse_step_rk4<M, R>(yt, s_time[k], ldt, PR, a.PD, FR, lam, gF, nullptr, 0);
+            if constexpr (AdjointShape<R>::lockstep)
+                __syncthreads();
         }
     }
     if (!active)
@@ -484,9 +509,7 @@ adjoint_kernel(const __grid_constant__ AdjointArgs<M, T> a)
 // through the whole trajectory, so the job runs in waves of (resident blocks
 // x SMs) blocks and its time is about waves x resident warps per SM.  Choose
 // the multiple of 32 (<= AdjointShape<T>::block) minimising that product (ties:
-// the larger block) -- e.g. for 65,536 nodes on 148 SMs with two blocks per
-// SM: 112 threads (two nearly full waves) instead of 128 (a second wave on
-// 108 of 148 SMs).  A grid below one wave counts the blocks it puts on an SM,
+// the larger block).  A grid below one wave counts the blocks it puts on an SM,
 // not those that would fit: 2,001 nodes in FP64 take blocks of 32 (one warp on
 // each of 63 SMs) instead of 256 (eight on each of 8): GRL1 100 steps 1.80 ->
 // 1.13 ms, 8,000 nodes (blocks of 64) 1.87 -> 1.19 ms.
@@ -528,6 +551,8 @@ inline int launch_adjoint_t(const goss_adjoint_launch* L)
     a.scratch = static_cast<T*>(L->scratch);
     a.tape = static_cast<T*>(L->tape);
     a.taped_segments = L->taped_segments;
+    if (L->keep_stages && (S != Explicit::RK4 || sizeof(T) != 8))
+        return GOSS_ERR_ARGUMENT;
     a.fparams_bar = L->field_params_bar;
     a.states_bar = L->states_bar;
     a.flags = L->flags;
@@ -567,7 +592,11 @@ inline int launch_adjoint_t(const goss_adjoint_launch* L)
         if (block == 0 || block > AdjointShape<R>::block || block % 32)
             return GOSS_ERR_ARGUMENT;
         const unsigned grid = (L->num_nodes + block - 1) / block;
-        adjoint_kernel<M, T, S, R><<<grid, block, shm, (cudaStream_t)L->stream>>>(a);
+        constexpr bool can_keep = S == Explicit::RK4 && sizeof(T) == 8;
+        if (can_keep && L->keep_stages)
+            adjoint_kernel<M, T, S, R, can_keep><<<grid, block, shm, (cudaStream_t)L->stream>>>(a);
+        else
+            adjoint_kernel<M, T, S, R><<<grid, block, shm, (cudaStream_t)L->stream>>>(a);
     }
     return cudaPeekAtLastError() == cudaSuccess ? 0 : GOSS_ERR_CUDA;
 }

@@ -510,12 +510,21 @@ __device__ __forceinline__ void grl_update(Acc<float>* y, float* yt, const float
     }
 }
 
+struct KeepNothing {
+    template <typename T>
+    __device__ __forceinline__ void operator()(int, const T*) const
+    {
+    }
+};
+
 // One internal step of an explicit solver at time lt with step ldt, in place
 // on the accumulated states (shared by the solver kernels and the adjoint
 // kernels' record and recompute passes, so all take identical arithmetic).
-template <class M, typename T, Explicit S>
+// keep(stage, k) sees RK4's stage derivatives.
+template <class M, typename T, Explicit S, class Keep = KeepNothing>
 __device__ __forceinline__ void explicit_step(Acc<T>* y, const double lt, const double ldt, const T* __restrict__ P,
-                                              const double* __restrict__ PD, const T* __restrict__ F, const T delta)
+                                              const double* __restrict__ PD, const T* __restrict__ F, const T delta,
+                                              Keep keep = Keep())
 {
     constexpr int n = M::num_states;
     const T h = T(ldt);
@@ -543,6 +552,7 @@ __device__ __forceinline__ void explicit_step(Acc<T>* y, const double lt, const 
         for (int st = 0; st < 4; ++st) {
             T k[n];
             model_rhs<M, T>(yt, st == 0 ? lt : st == 3 ? lt + ldt : lt + 0.5 * ldt, P, PD, F, k);
+            keep(st, k);
             const T w = st == 1 || st == 2 ? T(2.0) : T(1.0), c = st == 2 ? h : hh;
 #pragma unroll
             for (int i = 0; i < n; ++i) {

@@ -208,6 +208,10 @@ typedef struct goss_adjoint_launch {
                                   GOSS_FP32 (GRL1): the FP32 trajectory (its
                                   checkpoints, tape and recomputed steps)
                                   differentiated in FP64 */
+    int32_t keep_stages;      /* GOSS_RK4 in GOSS_FP64: the recompute keeps the
+                                 first three stage derivatives of every step in
+                                 scratch, which then holds 4 n rows per step
+                                 instead of n */
 } goss_adjoint_launch;
 
 /* A compiled model: produced by the code generator for one .ode model and one

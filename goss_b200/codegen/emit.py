@@ -27,6 +27,7 @@ from .ir import CONST, FIELD, STATE, TIME_CLS, Assign, ModelIR, Output, Program,
 from .odeparse import TIME
 from .ad import ReverseProgram
 from .factor import factor_common
+from .groups import declarations
 from .hoist import ConstantFolder
 from .printer import CPrinter, c_double
 from .sparse import LUStructure
@@ -802,7 +803,8 @@ class ModelSource:
         L.append("  template <typename T>")
         L.append(f"  __device__ static __forceinline__ void linearized_split({sig}, T* __restrict__ linear, T* __restrict__ rhs)")
         L.append("  {")
-        L += ["    " + x for x in head + self._dev_split_lines(lin_full, {"linear": "linear", "rhs": "rhs"})]
+        linearized_lines = head + self._dev_split_lines(lin_full, {"linear": "linear", "rhs": "rhs"})
+        L += ["    " + x for x in linearized_lines]
         L.append("    (void)time; (void)P; (void)PD; (void)F;")
         L.append("  }")
         L.append("")
@@ -810,9 +812,12 @@ class ModelSource:
         L.append("  template <typename T>")
         L.append(f"  __device__ static __forceinline__ void rhs_split({sig}, T* __restrict__ values)")
         L.append("  {")
-        L += ["    " + x for x in head + self._dev_split_lines(self.rhs, {"values": "values"})]
+        rhs_split_lines = head + self._dev_split_lines(self.rhs, {"values": "values"})
+        L += ["    " + x for x in rhs_split_lines]
         L.append("    (void)time; (void)P; (void)PD; (void)F;")
         L.append("  }")
+        L.append("")
+        L += declarations(linearized_lines, rhs_split_lines, len(self.states))
         L.append("")
         L.append("  // forward-difference Jacobian of rhs_split at y into the packed Newton matrix (structural")
         L.append("  // entries; fd_clear sets the others): f1 = f(y, time); column i recomputes only the")

@@ -631,6 +631,98 @@ __device__ __forceinline__ void explicit_step(Acc<T>* y, const double lt, const 
     }
 }
 
+// A step of 32 nodes by the four warps of a block, one lane of each warp to a
+// node: warp W evaluates and updates the states of its row group
+// (M::linear_group, M::rhs_group: the rows dealt out by the cost of what each
+// needs), and what only the other rows need falls out of its copy of the
+// model's program.  All warps hold all states; share(values) exchanges the new
+// ones.  For grids that leave SMs idle, see explicit_in_groups.
+template <class M, Explicit S>
+__host__ __device__ constexpr int row_group(int i)
+{
+    return S == Explicit::GRL1 ? M::linear_group(i) : M::rhs_group(i);
+}
+template <class M, Explicit S, int W>
+__host__ __device__ constexpr int group_size()
+{
+    int c = 0;
+    for (int i = 0; i < M::num_states; ++i)
+        c += row_group<M, S>(i) == W;
+    return c;
+}
+
+template <class M, Explicit S, int W>
+__device__ __forceinline__ void grl_update_group(Acc<double>* y, const double* lin, const double* rhs, double h,
+                                                 double delta)
+{
+    constexpr int n = M::num_states, N = group_size<M, S, W>();
+    if constexpr (N > 0) {
+        Acc<double> u[N];
+        double a[N], b[N];
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i)
+            if (row_group<M, S>(i) == W) {
+                u[c] = y[i];
+                a[c] = lin[i];
+                b[c] = rhs[i];
+                ++c;
+            }
+        grl_update<N, false>(u, a, a, b, h, delta);
+        c = 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i)
+            if (row_group<M, S>(i) == W)
+                y[i] = u[c++];
+    }
+}
+
+template <class M, Explicit S, int W, class Share>
+__device__ __forceinline__ void group_step(Acc<double>* y, const double lt, const double h, const double* __restrict__ P,
+                                           const double* __restrict__ PD, const double* __restrict__ F,
+                                           const double delta, Share share)
+{
+    constexpr int n = M::num_states;
+    const double hh = 0.5 * h;
+    double yt[n];
+#pragma unroll
+    for (int i = 0; i < n; ++i)
+        yt[i] = y[i].value();
+    if constexpr (S == Explicit::RK4) {
+        double sum[n];
+#pragma unroll 1
+        for (int st = 0; st < 4; ++st) {
+            double k[n];
+            model_rhs<M, double>(yt, st == 0 ? lt : st == 3 ? lt + h : lt + 0.5 * h, P, PD, F, k);
+            const double w = st == 1 || st == 2 ? 2.0 : 1.0, c = st == 2 ? h : hh;
+#pragma unroll
+            for (int i = 0; i < n; ++i)
+                if (row_group<M, S>(i) == W) {
+                    sum[i] = st == 0 ? k[i] : sum[i] + w * k[i];
+                    if (st == 3) {
+                        y[i].add(double(models::F64(h * sum[i]) / models::F64(6.0)));
+                        yt[i] = y[i].value();
+                    } else {
+                        yt[i] = y[i].plus(c * k[i]);
+                    }
+                }
+            share(yt);
+        }
+    } else {
+        static_assert(S == Explicit::GRL1, "unhandled explicit solver");
+        double lin[n], rhs[n];
+        model_linearized<M, double>(yt, lt, P, PD, F, lin, rhs);
+        grl_update_group<M, S, W>(y, lin, rhs, h, delta);
+#pragma unroll
+        for (int i = 0; i < n; ++i)
+            yt[i] = y[i].value();
+        share(yt);
+    }
+#pragma unroll
+    for (int i = 0; i < n; ++i)
+        y[i].load(yt[i]);
+}
+
 // Advance one node over nsteps internal steps of one explicit solver, from
 // its accumulated states and field parameters, and store the result.
 template <class M, typename T, Explicit S>
@@ -815,6 +907,132 @@ __global__ void __launch_bounds__(128, Blocks) schedule_kernel(const __grid_cons
         a.node_status[node] |= GOSS_FLAG_NONFINITE;
         atomicOr(a.flags, GOSS_FLAG_NONFINITE);
     }
+}
+
+// a barrier of the block's 128 threads that its warps reach at different places
+__device__ __forceinline__ void block_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+// schedule_kernel with the rows of a node split over the block's four warps (W:
+// this warp's).  A thread alone on its scheduler is bound by the length of its
+// instruction stream; here that is a third of the step's (TP06's four groups
+// cost 1.3 times the whole between them).  One exchange through shared memory
+// and one barrier per model evaluation.
+template <class M, Explicit S, int W>
+__device__ __forceinline__ void group_node(const ExplicitArgs<M, double>& a, double (*shared)[M::num_states][32])
+{
+    constexpr int n = M::num_states;
+    const uint32_t lane = threadIdx.x & 31, at = blockIdx.x * 32 + lane;
+    const bool active = at < a.N;
+    const uint32_t node = active ? at : a.N - 1;
+    Acc<double> y[n];
+    double* const v = a.vector ? a.vector + (uint64_t)a.dofs[node] * a.num_fields : nullptr;
+#pragma unroll
+    for (int i = 0; i < n; ++i)
+        y[i].load(v && a.field_of[i] >= 0 ? v[a.field_of[i]] : a.states[i * a.ld + node]);
+    double F[Dims<M>::nfp];
+    load_field<M, double>(a.fparams, a.ld, node, F);
+    block_barrier();  // every warp has read the states the others will write
+    unsigned turn = 0;
+    // two buffers in turn: a warp is at most one barrier ahead of the others
+    const auto share = [&](double* values) {
+        double(*const s)[32] = shared[turn];
+        turn ^= 1;
+#pragma unroll
+        for (int i = 0; i < n; ++i)
+            if (row_group<M, S>(i) == W)
+                s[i][lane] = values[i];
+        block_barrier();
+#pragma unroll
+        for (int i = 0; i < n; ++i)
+            if (row_group<M, S>(i) != W)
+                values[i] = s[i][lane];
+    };
+    double lt = a.t, ldt = a.ldt;
+    uint64_t nsteps = a.nsteps;
+    bool finite = true;
+    for (uint32_t f = 0; f < a.forwards; ++f) {
+        if (a.schedule) {
+            lt = a.schedule[f].t;
+            ldt = a.schedule[f].ldt;
+            nsteps = a.schedule[f].nsteps;
+        }
+        for (uint64_t step = 0; step < nsteps; ++step) {
+            group_step<M, S, W>(y, lt, ldt, a.P, a.PD, F, a.delta, share);
+            lt += ldt;
+        }
+        if (a.out && active) {
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+                if (row_group<M, S>(i) != W)
+                    continue;
+                const double w = y[i].store();
+                finite = finite && isfinite(w);
+                if (a.field_of[i] >= 0) {
+                    const uint64_t k = (uint64_t)a.field_of[i], row = (uint64_t)f * a.num_fields;
+                    a.out[a.tangled ? row * a.N + (uint64_t)node * a.num_fields + k : (row + k) * a.N + node] = w;
+                }
+            }
+        }
+    }
+    if (!active)
+        return;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+        if (row_group<M, S>(i) != W)
+            continue;
+        const double w = y[i].store();
+        a.states[i * a.ld + node] = w;
+        if (v && a.field_of[i] >= 0)
+            v[a.field_of[i]] = w;
+        finite = finite && isfinite(w);
+    }
+    if (!finite) {
+        a.node_status[node] |= GOSS_FLAG_NONFINITE;  // every warp writes the same value
+        atomicOr(a.flags, GOSS_FLAG_NONFINITE);
+    }
+}
+
+template <class M, Explicit S>
+__global__ void __launch_bounds__(128, 2) group_kernel(const __grid_constant__ ExplicitArgs<M, double> a)
+{
+    __shared__ double shared[2][M::num_states][32];
+    switch (threadIdx.x >> 5) {
+    case 0: group_node<M, S, 0>(a, shared); break;
+    case 1: group_node<M, S, 1>(a, shared); break;
+    case 2: group_node<M, S, 2>(a, shared); break;
+    default: group_node<M, S, 3>(a, shared); break;
+    }
+}
+
+// Models generated without row groups, with too few states to share out (or too
+// many for the exchange buffers) keep a thread per node.  So does GRL2: a copy
+// of the program that leaves out rows contracts other products, and over 100 ms
+// of 2,048 nodes GRL2 carried that to 1.6e-9 of the reference (bar 1e-9).
+template <class M, class = void>
+struct HasRowGroups {
+    static constexpr bool value = false;
+};
+template <class M>
+struct HasRowGroups<M, decltype(void(M::linear_group(0) + M::rhs_group(0)))> {
+    static constexpr bool value = M::num_states > 8 && M::num_states <= 64;
+};
+template <class M, typename T, Explicit S>
+constexpr bool explicit_groups =
+    sizeof(T) == 8 && (S == Explicit::GRL1 || S == Explicit::RK4) && HasRowGroups<M>::value;
+
+// Whether to split the rows: blocks of 32 nodes on at most half the SMs.  The
+// time is flat to a quarter of them, then grows by the block as the SMs of a
+// GPC fetch four instruction streams each through one cache.  TP06, 100 steps,
+// thread per node / split, ms (4 fields, FP64):
+//   nodes      256          1,184        1,792        2,368        3,840
+//   GRL1  0.425 / 0.203  0.494 / 0.226  0.488 / 0.338  0.499 / 0.404  0.483 / 0.595
+//   RK4   1.340 / 0.710  1.511 / 0.763  1.512 / 1.164  1.546 / 1.392  1.558 / 2.079
+inline bool explicit_in_groups(uint32_t num_nodes)
+{
+    int dev = 0, sms = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+           num_nodes <= 16u * (uint32_t)sms;
 }
 
 // ---------------------------------------------------------------------------
@@ -1688,6 +1906,12 @@ inline int launch_explicit(const goss_launch* L)
     const cudaStream_t st = (cudaStream_t)L->stream;
     const bool wide = explicit_two_shapes<T, S> && block == 128 && explicit_blocks(grid) == 2;
     constexpr int wide_blocks = explicit_two_shapes<T, S> ? 2 : ExplicitMinBlocks<T>::value;
+    if constexpr (explicit_groups<M, T, S>) {
+        if (block == 128 && explicit_in_groups(L->num_nodes)) {
+            group_kernel<M, S><<<(L->num_nodes + 31) / 32, 128, 0, st>>>(a);
+            return cudaPeekAtLastError() == cudaSuccess ? 0 : GOSS_ERR_CUDA;
+        }
+    }
     if (L->schedule || L->vector) {
         if constexpr (explicit_extended<S>) {
             if (wide)

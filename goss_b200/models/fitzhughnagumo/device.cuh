@@ -156,6 +156,10 @@ struct M_fitzhughnagumo {
     (void)time; (void)P; (void)PD; (void)F;
   }
 
+  // the rows of linearized_split and of rhs_split dealt to the four warps of a block
+  __host__ __device__ static constexpr int linear_group(int i) { return "01"[i] - '0'; }
+  __host__ __device__ static constexpr int rhs_group(int i) { return "01"[i] - '0'; }
+
   // forward-difference Jacobian of rhs_split at y into the packed Newton matrix (structural
   // entries; fd_clear sets the others): f1 = f(y, time); column i recomputes only the
   // statements of its rows that depend on state i

@@ -942,9 +942,9 @@ def measured_peaks(dev):
 
 # FP64-pipe instructions per TP06 GRL1 cell-step of explicit_kernel<TP06, double,
 # GRL1> (split program): the thread-level dadd + dmul + dfma counts of one ncu
-# capture of `bench.py --profile double --steps 1 --warmup 1 --nodes 262144`
-# divided by the cell-steps of the launch (262,144 x 1000)
-FP64_PIPE_OPS_PER_CELL_STEP = 1962.0  # dadd 262 + dmul 371 + dfma 1329 (B200, ncu)
+# capture of `bench.py --profile double --steps 1 --warmup 1 --nodes 56832`
+# divided by the cell-steps of the launch (56,832 x 1000)
+FP64_PIPE_OPS_PER_CELL_STEP = 1737.0  # dadd 200 + dmul 437 + dfma 1100 (B200, ncu)
 
 
 def roofline_fp64(value_fp64, peaks):
@@ -977,7 +977,8 @@ def roofline(md, value_fp32, ms_per_step, n_nodes, peaks=None):
     polynomial on the FP32 pipe for |a h| < 1/4, ex2 and a reciprocal above;
     ncu counts 131 XU instructions per TP06 step in all, against 129 here).
     FP32-pipe ops: adds, muls, the multiply of every division and exponential,
-    and ~10 ops of the phi1 update per state."""
+    and ~10 ops of the phi1 update per state; a fused multiply-add counts as two,
+    so this share can exceed 1."""
     census = md["op_census"]
     lin = census.get("linearized_split", census["linearized"])
     n = len(md["state_names"])

@@ -61,9 +61,9 @@ struct BatchArgs : BatchParamsT<T> {
 // population's states through HBM, and with all forwards in one launch it is
 // bound by instruction issue, and in both cases warps in flight matter --
 // measured on B200 (1.97M-node mix, 1000 fused one-step forwards): 2 blocks
-// 128 ms, 3 blocks 98 ms, 4 blocks 90 ms, 5 blocks 92 ms, 6 blocks 99 ms.  FP64
-// stays at the compiler's choice (its models spill heavily below ~240
-// registers).
+// 128 ms, 3 blocks 98 ms, 4 blocks 90 ms, 5 blocks 92 ms, 6 blocks 99 ms (4
+// blocks 74.5 ms since the update and the rounding are packed).  FP64 stays at
+// the compiler's choice (its models spill heavily below ~240 registers).
 #ifndef GOSS_BATCH_MIN_BLOCKS_F32
 #define GOSS_BATCH_MIN_BLOCKS_F32 4
 #endif

@@ -7,9 +7,10 @@
 // travel in the kernel's parameter block (constant bank, read as free
 // operands); per-node field parameters are loaded once into registers.
 //
-// Each kernel restates the arithmetic of one reference solver; the FP64
-// instantiation follows the reference operation order so that it agrees with
-// the FP64 CPU oracle to rounding.
+// Each kernel restates the arithmetic of one reference solver.  The FP64
+// instantiations evaluate the model with common factors pulled out and every
+// distinct exponential and reciprocal once, so they agree with the FP64 CPU
+// oracle to rounding; GOSS_FP64_PRINTED keeps the reference's own order.
 //
 //   explicit_kernel<M, T, ExplicitEuler>  cpp/goss/ExplicitEuler.cpp:64-87
 //   explicit_kernel<M, T, RK4>            cpp/goss/RK4.cpp:68-102
@@ -132,44 +133,9 @@ __device__ __forceinline__ void load_field(const double* __restrict__ fp, uint64
 
 // GRL increment of one state, FP64, in the reference's own expression
 // b/a*(exp(a*h) - 1.0) or b*h (GRL1.h:80-83)
-__device__ __forceinline__ double grl_increment_printed(double a, double b, double h, double delta)
+__device__ __forceinline__ double grl_increment(double a, double b, double h, double delta)
 {
     return (fabs(a) > delta) ? b / a * (exp(a * h) - 1.0) : b * h;
-}
-
-// coefficients up to this size take the Euler increment whatever delta is:
-// their reciprocal could overflow
-constexpr double kGrlTiny = 0x1p-1000;
-
-// The same expression for N states at once, with branch-free arithmetic.
-// e^x - 1 keeps the rounding of e^x to a double (its cancellation is part of
-// the reference's results: the exact (e^x - 1)/x, cheaper and more accurate,
-// differed from them by up to 1.4e-10 of V through an upstroke).  For
-// |x| < 1/8 -- gates slower than 8 h, nearly all states of a cardiac model at
-// its usual step -- e^x is 1 + x phi1(x) in one FMA over a polynomial, beyond
-// that f64_exp, under one branch for the N states so that their polynomials
-// and reciprocals overlap.
-template <int N>
-__device__ __forceinline__ void grl_increments(const double* a, const double* b, double h, double delta, double* inc)
-{
-    double x[N], e[N];
-    int far = 0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        x[i] = a[i] * h;
-        e[i] = fma(x[i], models::f64_phi1_small(x[i]), 1.0);
-        inc[i] = b[i] * models::f64_rcp(a[i]);
-        far = max(far, __double2hiint(x[i]) & 0x7fffffff);
-    }
-    if (far >= 0x3fc00000) {  // |x| >= 1/8, infinite or NaN
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-            if ((__double2hiint(x[i]) & 0x7fffffff) >= 0x3fc00000)
-                e[i] = models::f64_exp(x[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-        inc[i] = fabs(a[i]) > delta ? inc[i] * (e[i] - 1.0) : b[i] * h;
 }
 
 // GRL increment of one state, FP32: b*h*phi1(a*h), algebraically identical
@@ -395,11 +361,12 @@ struct NodeIO {
 // distinct transcendental and reciprocal of a state-dependent operand
 // evaluated once), in FP32 and in FP64.  The split FP64 programs change the
 // reference's results by re-association only; they stay within 1e-10 of the
-// reference over 10^5 TP06 GRL1 steps.  Printed = true takes the programs in
+// reference over 10^5 TP06 GRL1 steps.  GRL1Printed takes the programs in
 // the printed operation order of the model (one exp per occurrence, divisions
 // as written), the arithmetic of the reference's own generated code.
 // Split FP64 programs run on models::F64, a double whose division,
-// exponentials and square root have no branches (goss_device_math.cuh).
+// exponentials and square root have no branches (goss_device_math.cuh), but
+// those of GRL1 and GRL2, see grl_linearized.
 template <typename T>
 struct SplitScalar {
     using type = T;
@@ -422,15 +389,12 @@ __device__ __forceinline__ split_t<T>* as_split(T* p)
     return reinterpret_cast<split_t<T>*>(p);
 }
 
-template <class M, typename T, bool Printed = false>
+template <class M, typename T>
 __device__ __forceinline__ void model_linearized(const T* y, double t, const T* P, const double* PD, const T* F,
                                                  T* lin, T* rhs)
 {
-    if constexpr (Printed)
-        M::template linearized<T>(y, t, P, PD, F, lin, rhs);
-    else
-        M::template linearized_split<split_t<T>>(as_split(y), t, as_split(P), PD, as_split(F), as_split(lin),
-                                                 as_split(rhs));
+    M::template linearized_split<split_t<T>>(as_split(y), t, as_split(P), PD, as_split(F), as_split(lin),
+                                             as_split(rhs));
 }
 template <class M, typename T>
 __device__ __forceinline__ void model_rhs(const T* y, double t, const T* P, const double* PD, const T* F, T* f)
@@ -438,38 +402,38 @@ __device__ __forceinline__ void model_rhs(const T* y, double t, const T* P, cons
     M::template rhs_split<split_t<T>>(as_split(y), t, as_split(P), PD, as_split(F), as_split(f));
 }
 
-// The GRL update of every state: y[i].add(increment), or with Half the states
-// of the half step, yt[i] = y[i].plus(increment).  FP64: four states at a time
-// (TP06, 262,144 nodes x 100 steps: 2 / 4 / 7 / 10 / 19 at a time 3.78 / 3.76 /
-// 3.79 / 3.91 / 4.70 ms), each group's states updated at once.
-constexpr int kGrlStates = 4;
-
-template <int N, bool Half>
-__device__ __forceinline__ void grl_group(Acc<double>* y, double* yt, const double* lin, const double* rhs, double h,
-                                          double delta)
+// The linearised model of the GRL steps.  FP64: plain doubles with CUDA's own
+// division, exponentials and logarithms, whose rounding every result of the
+// solver carries.  Where a state's coefficient a crosses zero (V's does in
+// every upstroke) e^{ah} - 1 is a few multiples of 2^-53, so the last bit of a
+// decides 1e-8 of that node's increment: on models::F64 the evaluation takes
+// half the time (262,144 TP06 nodes x 100 steps 3.76 instead of 7.13 ms) but
+// moved single nodes by 5e-8 of the states' scale, no nearer to nor further
+// from the exact increment.
+template <class M, typename T, bool Printed = false>
+__device__ __forceinline__ void grl_linearized(const T* y, double t, const T* P, const double* PD, const T* F, T* lin,
+                                               T* rhs)
 {
-    double inc[N];
-    grl_increments<N>(lin, rhs, h, delta, inc);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        if constexpr (Half)
-            yt[i] = y[i].plus(inc[i]);
-        else
-            y[i].add(inc[i]);
-    }
+    if constexpr (Printed)
+        M::template linearized<T>(y, t, P, PD, F, lin, rhs);
+    else
+        M::template linearized_split<T>(y, t, P, PD, F, lin, rhs);
 }
 
+// The GRL update of every state: y[i].add(increment), or with Half the states
+// of the half step, yt[i] = y[i].plus(increment).
 template <int n, bool Half>
 __device__ __forceinline__ void grl_update(Acc<double>* y, double* yt, const double* lin, const double* rhs, double h,
                                            double delta)
 {
-    constexpr int N = kGrlStates, rest = n % N;
-    const double d = fmax(delta, kGrlTiny);
 #pragma unroll
-    for (int i = 0; i + N <= n; i += N)
-        grl_group<N, Half>(y + i, yt + i, lin + i, rhs + i, h, d);
-    if constexpr (rest != 0)
-        grl_group<rest, Half>(y + n - rest, yt + n - rest, lin + n - rest, rhs + n - rest, h, d);
+    for (int i = 0; i < n; ++i) {
+        const double d = grl_increment(lin[i], rhs[i], h, delta);
+        if constexpr (Half)
+            yt[i] = y[i].plus(d);
+        else
+            y[i].add(d);
+    }
 }
 
 // FP32: two states at a time in packed arithmetic, the increments and the
@@ -566,15 +530,13 @@ __device__ __forceinline__ void explicit_step(Acc<T>* y, const double lt, const 
     } else if constexpr (S == Explicit::GRL1) {
         // GRL1.h:72-84
         T lin[n], rhs[n];
-        model_linearized<M, T>(yt, lt, P, PD, F, lin, rhs);
+        grl_linearized<M, T>(yt, lt, P, PD, F, lin, rhs);
         grl_update<n, false>(y, yt, lin, rhs, h, delta);
     } else if constexpr (S == Explicit::GRL1Printed) {
         // GRL1.h:72-84 over the printed model program
         T lin[n], rhs[n];
-        model_linearized<M, T, true>(yt, lt, P, PD, F, lin, rhs);
-#pragma unroll
-        for (int i = 0; i < n; ++i)
-            y[i].add(grl_increment_printed(lin[i], rhs[i], h, delta));
+        grl_linearized<M, T, true>(yt, lt, P, PD, F, lin, rhs);
+        grl_update<n, false>(y, yt, lin, rhs, h, delta);
     } else if constexpr (S == Explicit::GRL2) {
         // GRL2: GRL2.cpp:78-82.  The reference's branch threshold is a
         // self-initialised local (GRL2.cpp:67) whose -O3 build behaves as 0:
@@ -584,7 +546,7 @@ __device__ __forceinline__ void explicit_step(Acc<T>* y, const double lt, const 
 #pragma unroll(sizeof(T) == 4 ? 2 : 1)
         for (int st = 0; st < 2; ++st) {
             T lin[n], rhs[n];
-            model_linearized<M, T>(yt, lt, P, PD, F, lin, rhs);
+            grl_linearized<M, T>(yt, lt, P, PD, F, lin, rhs);
             if (st == 0)
                 grl_update<n, true>(y, yt, lin, rhs, hh, T(0));
             else
@@ -642,6 +604,8 @@ __host__ __device__ constexpr int row_group(int i)
 {
     return S == Explicit::GRL1 ? M::linear_group(i) : M::rhs_group(i);
 }
+constexpr int kGrlStates = 4;  // states under one branch
+
 template <class M, Explicit S, int W>
 __host__ __device__ constexpr int group_size()
 {
@@ -651,29 +615,62 @@ __host__ __device__ constexpr int group_size()
     return c;
 }
 
+// GRL increments of N states at once, without branches but one for the N.
+// e^x - 1 keeps the rounding of e^x to a double, as the reference's expression
+// does (the exact (e^x - 1)/x, cheaper, differed from it by up to 1.4e-10 of V
+// through an upstroke).  For |x| < 1/8 -- gates slower than 8 h, nearly all
+// states of a cardiac model at its usual step -- e^x is 1 + x phi1(x) in one
+// FMA over a polynomial, beyond that f64_exp.
+template <int N>
+__device__ __forceinline__ void grl_increments(const double* a, const double* b, double h, double delta, double* inc)
+{
+    double x[N], e[N];
+    int far = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        x[i] = a[i] * h;
+        e[i] = fma(x[i], models::f64_phi1_small(x[i]), 1.0);
+        inc[i] = models::f64_div(b[i], a[i]);
+        far = max(far, __double2hiint(x[i]) & 0x7fffffff);
+    }
+    if (far >= 0x3fc00000) {  // |x| >= 1/8, infinite or NaN
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if ((__double2hiint(x[i]) & 0x7fffffff) >= 0x3fc00000)
+                e[i] = models::f64_exp(x[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        inc[i] = fabs(a[i]) > delta ? inc[i] * (e[i] - 1.0) : b[i] * h;
+}
+
+// the update of this warp's states
 template <class M, Explicit S, int W>
 __device__ __forceinline__ void grl_update_group(Acc<double>* y, const double* lin, const double* rhs, double h,
                                                  double delta)
 {
     constexpr int n = M::num_states, N = group_size<M, S, W>();
     if constexpr (N > 0) {
-        Acc<double> u[N];
-        double a[N], b[N];
+        double a[N], b[N], d[N];
         int c = 0;
 #pragma unroll
         for (int i = 0; i < n; ++i)
             if (row_group<M, S>(i) == W) {
-                u[c] = y[i];
                 a[c] = lin[i];
                 b[c] = rhs[i];
                 ++c;
             }
-        grl_update<N, false>(u, a, a, b, h, delta);
+        constexpr int rest = N % kGrlStates;
+#pragma unroll
+        for (int i = 0; i + kGrlStates <= N; i += kGrlStates)
+            grl_increments<kGrlStates>(a + i, b + i, h, delta, d + i);
+        if constexpr (rest != 0)
+            grl_increments<rest>(a + N - rest, b + N - rest, h, delta, d + N - rest);
         c = 0;
 #pragma unroll
         for (int i = 0; i < n; ++i)
             if (row_group<M, S>(i) == W)
-                y[i] = u[c++];
+                y[i].add(d[c++]);
     }
 }
 
@@ -808,11 +805,11 @@ constexpr bool explicit_two_shapes =
 
 // Resident blocks per SM to run `grid` FP64 blocks of 128 with: the time of the
 // full waves and of the last one under either register cap.  Time of a wave
-// with one, two (three) blocks on every SM, measured for TP06 GRL1, 100 steps:
-// 0.455, 0.604 ms at 255 registers, 0.484, 0.620, 0.848 ms at 168 (RK4 1.41,
-// 1.84 against 1.82, 2.13; GRL2 0.94, 1.24 against 1.12, 1.34).  E.g. one node
-// 2, 50,021 nodes 3 (0.85 against 1.12 ms), 65,536 nodes 2 (1.16 against
-// 1.34 ms), 262,144 nodes 3 (3.75 against 4.04 ms).
+// with one, two (three) blocks on every SM, measured for TP06 and 100 steps
+// (GRL2's are GRL1's to 2 % in proportion): e.g. GRL1 one node 2, 50,021 nodes 3
+// (1.49 against 2.16 ms), 65,536 nodes 2 (2.16 against 2.56 ms), 262,144 nodes 3
+// (6.74 against 7.41 ms).
+template <Explicit S>
 inline int explicit_blocks(unsigned grid)
 {
     int dev = 0, sms = 0;
@@ -823,7 +820,9 @@ inline int explicit_blocks(unsigned grid)
         const unsigned slots = k * (unsigned)sms, full = grid / slots, rest = grid % slots;
         return full * wave[k] + wave[(rest + sms - 1) / sms];
     };
-    constexpr double wide[] = {0.0, 0.455, 0.604}, narrow[] = {0.0, 0.484, 0.620, 0.848};
+    constexpr bool rk4 = S == Explicit::RK4;
+    constexpr double wide[] = {0.0, rk4 ? 1.81 : 1.007, rk4 ? 1.85 : 1.082};
+    constexpr double narrow[] = {0.0, rk4 ? 1.99 : 1.063, rk4 ? 2.14 : 1.149, rk4 ? 2.80 : 1.494};
     return time(2, wide) < time(3, narrow) ? 2 : 3;
 }
 
@@ -913,7 +912,10 @@ __global__ void __launch_bounds__(128, Blocks) schedule_kernel(const __grid_cons
 __device__ __forceinline__ void block_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // schedule_kernel with the rows of a node split over the block's four warps (W:
-// this warp's).  A thread alone on its scheduler is bound by the length of its
+// this warp's), the model on models::F64 for GRL1 too: a population of the size
+// that comes here has no node near enough to a coefficient's zero for that to
+// show (2,000 to 2,368 nodes through the stimulus: at most 7e-10 of the states'
+// scale between the two kernels; RK4's are equal bit for bit).  A thread alone on its scheduler is bound by the length of its
 // instruction stream; here that is a third of the step's (TP06's four groups
 // cost 1.3 times the whole between them).  One exchange through shared memory
 // and one barrier per model evaluation.
@@ -1025,10 +1027,16 @@ constexpr bool explicit_groups =
 // GPC fetch four instruction streams each through one cache.  TP06, 100 steps,
 // thread per node / split, ms (4 fields, FP64):
 //   nodes      256          1,184        1,792        2,368        3,840
-//   GRL1  0.425 / 0.203  0.494 / 0.226  0.488 / 0.338  0.499 / 0.404  0.483 / 0.595
+//   GRL1   1.00 / 0.203   1.05 / 0.226   1.05 / 0.338   1.09 / 0.404   1.04 / 0.595
 //   RK4   1.340 / 0.710  1.511 / 0.763  1.512 / 1.164  1.546 / 1.392  1.558 / 2.079
-inline bool explicit_in_groups(uint32_t num_nodes)
+// Coefficients within [-delta, delta] take the Euler increment; a delta below
+// kGrlTiny stays with the thread per node, whose division takes every operand.
+constexpr double kGrlTiny = 0x1p-1000;
+
+inline bool explicit_in_groups(uint32_t num_nodes, double delta)
 {
+    if (!(delta >= kGrlTiny))
+        return false;
     int dev = 0, sms = 0;
     return cudaGetDevice(&dev) == cudaSuccess &&
            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
@@ -1904,10 +1912,10 @@ inline int launch_explicit(const goss_launch* L)
     if (grid == 0)
         return 0;
     const cudaStream_t st = (cudaStream_t)L->stream;
-    const bool wide = explicit_two_shapes<T, S> && block == 128 && explicit_blocks(grid) == 2;
+    const bool wide = explicit_two_shapes<T, S> && block == 128 && explicit_blocks<S>(grid) == 2;
     constexpr int wide_blocks = explicit_two_shapes<T, S> ? 2 : ExplicitMinBlocks<T>::value;
     if constexpr (explicit_groups<M, T, S>) {
-        if (block == 128 && explicit_in_groups(L->num_nodes)) {
+        if (block == 128 && explicit_in_groups(L->num_nodes, S == Explicit::GRL1 ? a.delta : 1.0)) {
             group_kernel<M, S><<<(L->num_nodes + 31) / 32, 128, 0, st>>>(a);
             return cudaPeekAtLastError() == cudaSuccess ? 0 : GOSS_ERR_CUDA;
         }

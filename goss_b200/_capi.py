@@ -12,13 +12,13 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 RUNTIME_SO = PKG / "_lib" / "libgoss_b200.so"
 
-ABI_VERSION = 5
+ABI_VERSION = 6
 
 (GOSS_EXPLICIT_EULER, GOSS_RK4, GOSS_GRL1, GOSS_GRL2, GOSS_THETA, GOSS_ESDIRK23A, GOSS_RL1, GOSS_RL2, GOSS_RK2,
  GOSS_IMPLICIT_EULER) = range(10)
 GOSS_FP64, GOSS_FP32, GOSS_FP64_PRINTED = 0, 1, 2
 GOSS_OK, GOSS_ERR_ARGUMENT, GOSS_ERR_CUDA, GOSS_ERR_NEWTON, GOSS_ERR_UNSUPPORTED, GOSS_ERR_TIMEOUT = range(6)
-GOSS_FLAG_NONFINITE, GOSS_FLAG_NEWTON_FAILED, GOSS_FLAG_ITERATION_CAP = 1, 2, 4
+GOSS_FLAG_NONFINITE, GOSS_FLAG_NEWTON_FAILED, GOSS_FLAG_ITERATION_CAP, GOSS_FLAG_BAD_DOF = 1, 2, 4, 8
 
 SOLVER_KINDS = {
     "ExplicitEuler": GOSS_EXPLICIT_EULER,
@@ -153,8 +153,8 @@ _PROTOS = {
     "goss_system_get_solver_params": (C.c_int, [_sys, C.POINTER(SolverParams)]),
     "goss_system_forward": (C.c_int, [_sys, C.c_double, C.c_double]),
     "goss_system_forward_async": (C.c_int, [_sys, C.c_double, C.c_double]),
-    "goss_system_exchange_field_states": (C.c_int, [_sys, C.c_void_p, C.c_void_p, C.c_int32]),
-    "goss_system_step_field_states": (C.c_int, [_sys, C.c_double, C.c_double, C.c_void_p, C.c_void_p]),
+    "goss_system_exchange_field_states": (C.c_int, [_sys, C.c_void_p, C.c_uint64, C.c_void_p, C.c_int32]),
+    "goss_system_step_field_states": (C.c_int, [_sys, C.c_double, C.c_double, C.c_void_p, C.c_uint64, C.c_void_p]),
     "goss_system_synchronize": (C.c_int, [_sys]),
     "goss_system_solve": (C.c_int, [_sys, _dp, _dp, C.c_uint64, C.c_int32]),
     "goss_system_set_field_state_indices": (C.c_int, [_sys, _u32p, C.c_uint32]),

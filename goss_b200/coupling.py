@@ -123,14 +123,20 @@ class FieldStateCoupling:
         """Whether the exchange kernels can take ``v``'s memory as it is: a
         plain contiguous tensor of this device outside autograd (reverse and
         forward mode), at most 64 fields.  Anything else goes through torch's
-        own indexing."""
+        own indexing.  The entries of the maps are checked by the kernels."""
         import torch
         from torch.autograd import forward_ad
 
         return (type(v) is torch.Tensor and v.is_contiguous() and v.device == self.device and not v.requires_grad
                 and not v.is_neg() and self.num_fields <= 64 and forward_ad._current_level < 0
-                and all(d.dtype == torch.int64 and d.is_contiguous() and d.numel() == self.systems[lab].num_nodes
+                and all(type(d) is torch.Tensor and d.device == self.device and d.dtype == torch.int64
+                        and d.is_contiguous() and d.shape == (self.systems[lab].num_nodes,)
                         for lab, d in self.dofs.items()))
+
+    def _exchange(self, v, to_vector: int) -> None:
+        for lab, s in self.systems.items():
+            _capi.check(s._L.goss_system_exchange_field_states(s._h, v.data_ptr(), self.num_dofs,
+                                                               self.dofs[lab].data_ptr(), to_vector), s._h)
 
     def _touched(self, *tensors) -> None:
         """Tell autograd that the kernels wrote into these tensors."""
@@ -146,10 +152,9 @@ class FieldStateCoupling:
 
         v2 = self._vector(v)
         if self._plain(v):
-            for lab, s in self.systems.items():
-                _capi.check(s._L.goss_system_exchange_field_states(s._h, v.data_ptr(), self.dofs[lab].data_ptr(), 0),
-                            s._h)
-                self._touched(*self._views[lab])
+            self._exchange(v, 0)
+            for views in self._views.values():
+                self._touched(*views)
             return
         with torch.cuda.stream(self.stream):
             for lab, views in self._views.items():
@@ -164,9 +169,7 @@ class FieldStateCoupling:
 
         v2 = self._vector(v)
         if self._plain(v):
-            for lab, s in self.systems.items():
-                _capi.check(s._L.goss_system_exchange_field_states(s._h, v.data_ptr(), self.dofs[lab].data_ptr(), 1),
-                            s._h)
+            self._exchange(v, 1)
             self._touched(v)
             return
         with torch.cuda.stream(self.stream):
@@ -190,7 +193,7 @@ class FieldStateCoupling:
             # population by population: their dofs are disjoint
             for lab, s in self.systems.items():
                 _capi.check(s._L.goss_system_step_field_states(s._h, float(t0), float(t1) - float(t0), v.data_ptr(),
-                                                               self.dofs[lab].data_ptr()), s._h)
+                                                               self.num_dofs, self.dofs[lab].data_ptr()), s._h)
                 self._touched(*self._views[lab])
             self._touched(v)
             return

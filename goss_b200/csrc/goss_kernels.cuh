@@ -78,6 +78,7 @@ struct ExplicitArgs {
     double* out;
     double* vector;
     const int64_t* dofs;
+    uint64_t num_dofs;
     uint32_t num_fields;
     int32_t tangled;
     int8_t field_of[M::num_states];  // field of a state row, -1: none
@@ -844,6 +845,21 @@ template <Explicit S>
 constexpr bool explicit_extended =
     S == Explicit::Euler || S == Explicit::RK4 || S == Explicit::GRL1 || S == Explicit::GRL2;
 
+// A node's entry of the exchange vector; none without a vector, and none, with
+// the status flag set, for a dof outside it.
+template <class M, typename T>
+__device__ __forceinline__ double* exchange_entry(const ExplicitArgs<M, T>& a, uint32_t node)
+{
+    if (!a.vector)
+        return nullptr;
+    const uint64_t dof = (uint64_t)a.dofs[node];
+    if (dof < a.num_dofs)
+        return a.vector + dof * a.num_fields;
+    a.node_status[node] |= GOSS_FLAG_BAD_DOF;
+    atomicOr(a.flags, GOSS_FLAG_BAD_DOF);
+    return nullptr;
+}
+
 // One forward, or the forwards of a schedule with the states in registers from
 // one to the next (rounded between them as a store and load would); field
 // states from and to a vector and into outputs after every forward.  Saves a
@@ -858,7 +874,7 @@ __global__ void __launch_bounds__(128, Blocks) schedule_kernel(const __grid_cons
         return;
     Acc<T> y[n];
     {
-        const double* const v = a.vector ? a.vector + (uint64_t)a.dofs[node] * a.num_fields : nullptr;
+        const double* const v = exchange_entry(a, node);
 #pragma unroll
         for (int i = 0; i < n; ++i)
             y[i].load(v && a.field_of[i] >= 0 ? v[a.field_of[i]] : a.states[i * a.ld + node]);
@@ -893,7 +909,7 @@ __global__ void __launch_bounds__(128, Blocks) schedule_kernel(const __grid_cons
             }
         }
     }
-    double* const v = a.vector ? a.vector + (uint64_t)a.dofs[node] * a.num_fields : nullptr;
+    double* const v = exchange_entry(a, node);
 #pragma unroll
     for (int i = 0; i < n; ++i) {
         const double w = y[i].store();
@@ -927,7 +943,7 @@ __device__ __forceinline__ void group_node(const ExplicitArgs<M, double>& a, dou
     const bool active = at < a.N;
     const uint32_t node = active ? at : a.N - 1;
     Acc<double> y[n];
-    double* const v = a.vector ? a.vector + (uint64_t)a.dofs[node] * a.num_fields : nullptr;
+    double* const v = exchange_entry(a, node);
 #pragma unroll
     for (int i = 0; i < n; ++i)
         y[i].load(v && a.field_of[i] >= 0 ? v[a.field_of[i]] : a.states[i * a.ld + node]);
@@ -1895,6 +1911,7 @@ inline int launch_explicit(const goss_launch* L)
     a.out = L->out;
     a.vector = L->vector;
     a.dofs = L->dofs;
+    a.num_dofs = L->num_dofs;
     a.num_fields = L->num_fields;
     a.tangled = L->tangled;
     for (int i = 0; i < M::num_states; ++i)

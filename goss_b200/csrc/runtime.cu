@@ -104,10 +104,18 @@ struct FieldRows {
     uint32_t row[kMaxFields];
 };
 __global__ void exchange_kernel(double* __restrict__ states, uint64_t ld, uint32_t N, double* __restrict__ vec,
-                                const int64_t* __restrict__ dofs, const __grid_constant__ FieldRows f, int to_vector)
+                                uint64_t num_dofs, const int64_t* __restrict__ dofs,
+                                const __grid_constant__ FieldRows f, int to_vector, uint32_t* flags,
+                                uint8_t* node_status)
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        double* const v = vec + (uint64_t)dofs[i] * f.count;
+        const uint64_t dof = (uint64_t)dofs[i];
+        if (dof >= num_dofs) {
+            node_status[i] |= GOSS_FLAG_BAD_DOF;
+            atomicOr(flags, GOSS_FLAG_BAD_DOF);
+            continue;
+        }
+        double* const v = vec + dof * f.count;
         for (uint32_t k = 0; k < f.count; ++k) {
             double* const s = states + (uint64_t)f.row[k] * ld + i;
             if (to_vector)
@@ -325,6 +333,8 @@ int check_flags(goss_system* s, int64_t* totals = nullptr)
     }
     if (fresh & GOSS_FLAG_ITERATION_CAP)
         return fail(&s->last_error, GOSS_ERR_TIMEOUT, "a node exceeded the solver loop guard");
+    if (fresh & GOSS_FLAG_BAD_DOF)
+        return fail(&s->last_error, GOSS_ERR_ARGUMENT, "an entry of the dof map lies outside the exchange vector");
     return 0;
 }
 
@@ -1171,7 +1181,7 @@ int to_host(goss_system* s, double* host, const double* src, uint32_t k, const u
 }
 
 // enqueue one direction of an exchange with a device vector
-int exchange(goss_system* s, double* vec, const int64_t* dofs, int to_vector)
+int exchange(goss_system* s, double* vec, uint64_t num_dofs, const int64_t* dofs, int to_vector)
 {
     FieldRows f{};
     f.count = (uint32_t)s->fsi.size();
@@ -1180,23 +1190,25 @@ int exchange(goss_system* s, double* vec, const int64_t* dofs, int to_vector)
     if (f.count > kMaxFields)
         return fail(&s->last_error, GOSS_ERR_ARGUMENT, "more than %u field states", kMaxFields);
     std::copy(s->fsi.begin(), s->fsi.end(), f.row);
-    exchange_kernel<<<grid_for(s->N), 256, 0, s->stream>>>(s->d_states, s->ld, s->N, vec, dofs, f, to_vector);
+    exchange_kernel<<<grid_for(s->N), 256, 0, s->stream>>>(s->d_states, s->ld, s->N, vec, num_dofs, dofs, f, to_vector,
+                                                           s->d_flags, s->d_node_status);
     CUDA_TRY(s, cudaGetLastError());
     return 0;
 }
 
 }  // namespace
 
-GOSS_API int goss_system_exchange_field_states(goss_system* s, double* vector, const int64_t* dofs, int32_t to_vector)
+GOSS_API int goss_system_exchange_field_states(goss_system* s, double* vector, uint64_t num_dofs, const int64_t* dofs,
+                                               int32_t to_vector)
 {
     if (!s || !vector || !dofs)
         return fail(s ? &s->last_error : nullptr, GOSS_ERR_ARGUMENT, "NULL argument");
     int rc = set_device(s);
-    return rc ? rc : exchange(s, vector, dofs, to_vector);
+    return rc ? rc : exchange(s, vector, num_dofs, dofs, to_vector);
 }
 
 GOSS_API int goss_system_step_field_states(goss_system* s, double t, double interval, double* vector,
-                                           const int64_t* dofs)
+                                           uint64_t num_dofs, const int64_t* dofs)
 {
     if (!s || !vector || !dofs)
         return fail(s ? &s->last_error : nullptr, GOSS_ERR_ARGUMENT, "NULL argument");
@@ -1210,12 +1222,13 @@ GOSS_API int goss_system_step_field_states(goss_system* s, double t, double inte
         L.num_fields = (uint32_t)s->fsi.size();
         L.vector = vector;
         L.dofs = dofs;
+        L.num_dofs = num_dofs;
         return launch_forward(s, t, interval, L);
     }
-    rc = exchange(s, vector, dofs, 0);
+    rc = exchange(s, vector, num_dofs, dofs, 0);
     if (!rc)
         rc = launch_forward(s, t, interval);
-    return rc ? rc : exchange(s, vector, dofs, 1);
+    return rc ? rc : exchange(s, vector, num_dofs, dofs, 1);
 }
 
 GOSS_API int goss_system_set_field_state_indices(goss_system* s, const uint32_t* idx, uint32_t count)

@@ -35,7 +35,7 @@ extern "C" {
 #define GOSS_API
 #endif
 
-#define GOSS_B200_ABI_VERSION 5u
+#define GOSS_B200_ABI_VERSION 6u
 
 /* Solver kinds: the reference solver classes on this path. */
 enum goss_solver_kind {
@@ -78,7 +78,8 @@ enum goss_status {
 enum goss_flag_bits {
     GOSS_FLAG_NONFINITE = 1u,     /* a node produced a non-finite state */
     GOSS_FLAG_NEWTON_FAILED = 2u, /* a node's step size fell below min_dt */
-    GOSS_FLAG_ITERATION_CAP = 4u  /* a node exhausted the loop guard */
+    GOSS_FLAG_ITERATION_CAP = 4u, /* a node exhausted the loop guard */
+    GOSS_FLAG_BAD_DOF = 8u        /* a node's dof lies outside the exchange vector */
 };
 
 /* Solver parameters: the public members of the reference solver classes.
@@ -138,6 +139,7 @@ typedef struct goss_launch {
      * state rows before, and written there as well as to the rows after (device) */
     double* vector;
     const int64_t* dofs;
+    uint64_t num_dofs;       /* length of the vector: a node whose dof is not below it takes no part */
 } goss_launch;
 
 /* Batched evaluation of the model on device arrays (used by ODE.eval and the
@@ -378,18 +380,20 @@ GOSS_API int goss_system_device_states(goss_system* sys, double** states, uint64
 GOSS_API int goss_system_device_field_params(goss_system* sys, double** field_params, uint64_t* ld);
 GOSS_API int goss_system_set_stream(goss_system* sys, void* stream);
 GOSS_API int goss_system_forward_async(goss_system* sys, double t, double interval);
-/* Field states exchanged with a device vector of num_field_states values per
- * dof, vector[dofs[node]*num_field_states + k], dofs[num_nodes] on the device
- * (distinct, not checked here), enqueued on the system's stream without
+/* Field states exchanged with a device vector of num_dofs entries of
+ * num_field_states values, vector[dofs[node]*num_field_states + k],
+ * dofs[num_nodes] on the device, enqueued on the system's stream without
  * waiting: into the field states (to_vector 0) or into the vector (1); at most
- * 64 field states. */
-GOSS_API int goss_system_exchange_field_states(goss_system* sys, double* vector, const int64_t* dofs,
-                                               int32_t to_vector);
+ * 64 field states.  Two nodes must not share a dof (not checked).  A node whose
+ * dof lies outside [0, num_dofs) is left out; the next call that waits for the
+ * stream reports it (GOSS_FLAG_BAD_DOF, GOSS_ERR_ARGUMENT). */
+GOSS_API int goss_system_exchange_field_states(goss_system* sys, double* vector, uint64_t num_dofs,
+                                               const int64_t* dofs, int32_t to_vector);
 /* One step of an operator splitting (DOLFINODESystemSolver::step,
  * python/goss/dolfinutils.py:740-780): field states from the vector, forward,
  * field states to the vector, all enqueued. */
 GOSS_API int goss_system_step_field_states(goss_system* sys, double t, double interval, double* vector,
-                                           const int64_t* dofs);
+                                           uint64_t num_dofs, const int64_t* dofs);
 GOSS_API int goss_system_synchronize(goss_system* sys);
 
 /* Batched model evaluation on host arrays: states [count][n], times [count],

@@ -1201,7 +1201,7 @@ int exchange(goss_system* s, double* vec, uint64_t num_dofs, const int64_t* dofs
 GOSS_API int goss_system_exchange_field_states(goss_system* s, double* vector, uint64_t num_dofs, const int64_t* dofs,
                                                int32_t to_vector)
 {
-    if (!s || !vector || !dofs)
+    if (!s || (s->N && (!vector || !dofs)))
         return fail(s ? &s->last_error : nullptr, GOSS_ERR_ARGUMENT, "NULL argument");
     int rc = set_device(s);
     return rc ? rc : exchange(s, vector, num_dofs, dofs, to_vector);
@@ -1210,7 +1210,7 @@ GOSS_API int goss_system_exchange_field_states(goss_system* s, double* vector, u
 GOSS_API int goss_system_step_field_states(goss_system* s, double t, double interval, double* vector,
                                            uint64_t num_dofs, const int64_t* dofs)
 {
-    if (!s || !vector || !dofs)
+    if (!s || (s->N && (!vector || !dofs)))
         return fail(s ? &s->last_error : nullptr, GOSS_ERR_ARGUMENT, "NULL argument");
     int rc = set_device(s);
     if (rc)

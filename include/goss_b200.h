@@ -386,7 +386,8 @@ GOSS_API int goss_system_forward_async(goss_system* sys, double t, double interv
  * waiting: into the field states (to_vector 0) or into the vector (1); at most
  * 64 field states.  Two nodes must not share a dof (not checked).  A node whose
  * dof lies outside [0, num_dofs) is left out; the next call that waits for the
- * stream reports it (GOSS_FLAG_BAD_DOF, GOSS_ERR_ARGUMENT). */
+ * stream reports it (GOSS_FLAG_BAD_DOF, GOSS_ERR_ARGUMENT).  A system without
+ * nodes does nothing. */
 GOSS_API int goss_system_exchange_field_states(goss_system* sys, double* vector, uint64_t num_dofs,
                                                const int64_t* dofs, int32_t to_vector);
 /* One step of an operator splitting (DOLFINODESystemSolver::step,

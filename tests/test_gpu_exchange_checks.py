@@ -1,4 +1,5 @@
-"""The field-state exchange kernels on maps that changed after construction."""
+"""The field-state exchange kernels on maps that changed after construction and
+on empty populations."""
 from __future__ import annotations
 
 import numpy as np
@@ -71,3 +72,13 @@ def test_a_replaced_map_is_followed():
     d.step((0.0, 0.1), w)
     c.synchronize()
     assert (v == w).all()
+
+
+def test_an_empty_population_takes_no_part():
+    c, v = _coupling(nodes=(40, 0)), _vector()
+    for k in range(2):
+        c.step((0.1 * k, 0.1 * (k + 1)), v)
+    c.to_field_states(v)
+    c.from_field_states(v)
+    c.synchronize()
+    np.testing.assert_array_equal(v[c.dofs["0"]].cpu().numpy(), c.systems["0"].field_states[:, 0])

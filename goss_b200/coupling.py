@@ -120,18 +120,34 @@ class FieldStateCoupling:
         return v if v.dim() == 2 else v.view(-1, 1)
 
     def _plain(self, v) -> bool:
-        """Whether the exchange kernels can take ``v``'s memory as it is: a
-        plain contiguous tensor of this device outside autograd (reverse and
-        forward mode), at most 64 fields.  Anything else goes through torch's
-        own indexing.  The entries of the maps are checked by the kernels."""
+        """Whether the exchange kernels can take ``v``'s memory as it is: plain
+        contiguous tensors of this device, ``v`` and the field states outside
+        autograd (reverse and forward mode), function transforms, tracing and
+        the modes that observe torch's operations, at most 64 fields.  Anything
+        else goes through torch's own indexing.  The entries of the maps are
+        checked by the kernels."""
         import torch
         from torch.autograd import forward_ad
+        from torch.overrides import has_torch_function
+        from torch.utils._python_dispatch import is_in_torch_dispatch_mode
 
-        return (type(v) is torch.Tensor and v.is_contiguous() and v.device == self.device and not v.requires_grad
-                and not v.is_neg() and self.num_fields <= 64 and forward_ad._current_level < 0
-                and all(type(d) is torch.Tensor and d.device == self.device and d.dtype == torch.int64
-                        and d.is_contiguous() and d.shape == (self.systems[lab].num_nodes,)
-                        for lab, d in self.dofs.items()))
+        if (type(v) is not torch.Tensor or not v.is_contiguous() or v.device != self.device or v.is_neg()
+                or self.num_fields > 64 or torch.jit.is_tracing() or is_in_torch_dispatch_mode()
+                or has_torch_function((v,))):
+            return False
+        for lab, s in self.systems.items():
+            d = self.dofs[lab]
+            if not (type(d) is torch.Tensor and d.device == self.device and d.dtype == torch.int64
+                    and d.is_contiguous() and d.shape == (s.num_nodes,)):
+                return False
+        for x in (v, *(x for views in self._views.values() for x in views)):
+            if x.requires_grad or forward_ad.unpack_dual(x).tangent is not None:
+                return False
+        try:
+            v.data_ptr()
+        except RuntimeError:  # a function transform's wrapper has no memory of its own
+            return False
+        return True
 
     def _exchange(self, v, to_vector: int) -> None:
         for lab, s in self.systems.items():

@@ -1,5 +1,5 @@
-"""The field-state exchange kernels on maps that changed after construction and
-on empty populations."""
+"""The field-state exchange kernels on maps that changed after construction, on
+empty populations, and on vectors only torch's own operations can take."""
 from __future__ import annotations
 
 import numpy as np
@@ -82,3 +82,41 @@ def test_an_empty_population_takes_no_part():
     c.from_field_states(v)
     c.synchronize()
     np.testing.assert_array_equal(v[c.dofs["0"]].cpu().numpy(), c.systems["0"].field_states[:, 0])
+
+
+def test_transforms_and_modes_see_the_copies():
+    import torch
+    from torch.autograd import forward_ad
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    c = _coupling()
+
+    def read(v):
+        v = v.clone()
+        c.from_field_states(v)
+        return v
+
+    one = read(_vector())
+    assert torch.equal(torch.func.vmap(read)(_vector().repeat(3, 1)), one.repeat(3, 1))
+    seen = []
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    v = _vector()
+    with Watch():
+        c.from_field_states(v)
+    assert any("index_copy" in s for s in seen) and torch.equal(v, one)
+    with forward_ad.dual_level():
+        dual = forward_ad.make_dual(_vector(), torch.ones(80, dtype=torch.float64, device="cuda"))
+        assert not c._plain(dual) and c._plain(_vector())
+        c.from_field_states(dual)
+        owned = torch.cat([c.dofs["0"], c.dofs["1"]])
+        tangent = forward_ad.unpack_dual(dual).tangent
+        assert not tangent[owned].any() and tangent.sum() == 80 - owned.numel()
+    with torch.inference_mode():
+        v = _vector()
+        c.from_field_states(v)
+        assert torch.equal(v, one)

@@ -28,7 +28,11 @@ from .emit import ModelSource, c_ident, model_class_name
 from .ir import ModelIR
 from .odeparse import ODEModel
 
-GENERATOR_VERSION = "8"
+# of the generated text: a model compiled at run time is written again when it
+# was generated by another version
+GENERATOR_VERSION = "9"
+# of the key below, which names a model and its choices
+_KEY_VERSION = "8"
 
 _CENSUS_KEYS = ("add", "mul", "div", "exp", "log", "sqrt", "pow", "cmp", "misc")
 
@@ -49,7 +53,7 @@ def variant_id(model: ODEModel, field_parameters: Sequence[str] = (), monitored:
 
 def model_hash(model: ODEModel, field_parameters, monitored, linearization, jacobian: bool = False) -> str:
     h = hashlib.sha1()
-    h.update(GENERATOR_VERSION.encode())
+    h.update(_KEY_VERSION.encode())
     h.update(model.signature().encode())
     h.update(json.dumps(_key(field_parameters, monitored, linearization, jacobian)).encode())
     return h.hexdigest()

@@ -20,7 +20,7 @@ from typing import Dict, Optional, Sequence, Union
 from . import _capi
 from .build import build_variant
 from .codegen.odeparse import ODEModel, load_ode
-from .codegen.variant import model_hash, variant_id, write_variant
+from .codegen.variant import GENERATOR_VERSION, model_hash, variant_id, write_variant
 
 PKG = Path(__file__).resolve().parent
 JIT_DIR = PKG / "_jit"
@@ -139,7 +139,8 @@ def jit(model: Union[ODEModel, str, Path], field_parameters: Sequence[str] = (),
     ident = f"{ident}__{h[:10]}" if "__" not in ident else f"{ident}_{h[:10]}"
     vdir = JIT_DIR / ident
     with _lock:
-        if not (vdir / "model.json").exists() or json.loads((vdir / "model.json").read_text()).get("hash") != h:
+        meta = json.loads((vdir / "model.json").read_text()) if (vdir / "model.json").exists() else {}
+        if meta.get("hash") != h or meta.get("generator_version") != GENERATOR_VERSION:
             write_variant(model, vdir, field_parameters=field_parameters, monitored=monitored,
                           linearization=linearization, ident=ident, jacobian=jacobian)
     return load_variant(vdir)

@@ -27,7 +27,7 @@ from .ir import CONST, FIELD, STATE, TIME_CLS, Assign, ModelIR, Output, Program,
 from .odeparse import TIME
 from .ad import ReverseProgram
 from .factor import factor_common
-from .groups import declarations
+from .groups import MAX_ROWS, MIN_ROWS, declarations
 from .hoist import ConstantFolder
 from .printer import CPrinter, c_double
 from .sparse import LUStructure
@@ -638,10 +638,9 @@ class ModelSource:
         lines.append("}")
         return lines
 
-    def _dev_fd_jacobian_lines(self, with_rhs: bool = False, with_t0: bool = False,
-                               select: bool = False) -> List[str]:
-        """Body of ``fd_jacobian``: the forward-difference Jacobian of the split
-        right-hand side into the packed Newton matrix.  The unperturbed
+    def _dev_fd_jacobian_lines(self, with_t0: bool = False, select: bool = False) -> List[str]:
+        """Body of ``rhs_fd_jacobian``: f(y) and the forward-difference Jacobian of
+        the split right-hand side into the packed Newton matrix.  The unperturbed
         statements are evaluated once; column i then recomputes, for
         y + delta_i e_i, only the statements of its structural rows that depend
         on state i (the others keep their unperturbed values, which is what
@@ -678,11 +677,10 @@ class ModelSource:
                 lines.append(f"const double v_{b.name} = {prD(b.expr)};")
             else:
                 lines.append(f"const T v_{b.name} = {prT(factor_common(b.expr))};")
-        if with_rhs:  # f1 = f(y): the outputs of rhs_split, from the same statements
-            for r in range(n):
-                lines.append(f"f1[{r}] = {prT(factor_common(outs[r].expr)) if r in outs else 'T(0.0)'};")
-            if with_t0:
-                lines += self._t0_lines(binds, outs, prT, prD)
+        for r in range(n):  # f1 = f(y): the outputs of rhs_split, from the same statements
+            lines.append(f"f1[{r}] = {prT(factor_common(outs[r].expr)) if r in outs else 'T(0.0)'};")
+        if with_t0:
+            lines += self._t0_lines(binds, outs, prT, prD)
         if select:  # the columns only if want_jac (J is left as it is otherwise)
             lines += ["if (want_jac) {", "fd_clear(J);"]
         for i in range(n):
@@ -817,18 +815,9 @@ class ModelSource:
         L.append("    (void)time; (void)P; (void)PD; (void)F;")
         L.append("  }")
         L.append("")
-        L += declarations(linearized_lines, rhs_split_lines, len(self.states))
-        L.append("")
-        L.append("  // forward-difference Jacobian of rhs_split at y into the packed Newton matrix (structural")
-        L.append("  // entries; fd_clear sets the others): f1 = f(y, time); column i recomputes only the")
-        L.append("  // statements of its rows that depend on state i")
-        L.append("  template <typename T, class A>")
-        L.append(f"  __device__ static __forceinline__ void fd_jacobian({sig}, const T* __restrict__ f1, A J)")
-        L.append("  {")
-        L += ["    " + x for x in head + self._dev_fd_jacobian_lines()]
-        L.append("    (void)time; (void)P; (void)PD; (void)F; (void)f1; (void)J;")
-        L.append("  }")
-        L.append("")
+        if MIN_ROWS <= len(self.states) <= MAX_ROWS:
+            L += declarations(linearized_lines, rhs_split_lines, len(self.states))
+            L.append("")
         if self.jac is not None:
             L.append("  // f1 = f(y, time) (rhs_split) and the analytic Jacobian into the packed Newton matrix,")
             L.append("  // sharing their exponentials, reciprocals and intermediates")
@@ -858,11 +847,13 @@ class ModelSource:
             L.append("    (void)time; (void)t0; (void)P; (void)PD; (void)F; (void)f0; (void)f1; (void)J;")
             L.append("  }")
             L.append("")
-        L.append("  // the same, also writing f1 = f(y, time) (rhs_split) from its unperturbed statements")
+        L.append("  // forward-difference Jacobian of rhs_split at y into the packed Newton matrix (structural")
+        L.append("  // entries; fd_clear sets the others); column i recomputes only the statements of its rows")
+        L.append("  // that depend on state i.  f1 = f(y, time) (rhs_split) from the unperturbed statements")
         L.append("  template <typename T, class A>")
         L.append(f"  __device__ static __forceinline__ void rhs_fd_jacobian({sig}, T* __restrict__ f1, A J)")
         L.append("  {")
-        L += ["    " + x for x in head + self._dev_fd_jacobian_lines(with_rhs=True)]
+        L += ["    " + x for x in head + self._dev_fd_jacobian_lines()]
         L.append("    (void)time; (void)P; (void)PD; (void)F; (void)f1; (void)J;")
         L.append("  }")
         L.append("")
@@ -872,7 +863,7 @@ class ModelSource:
         L.append(f"  __device__ static __forceinline__ void rhs_fd_jacobian_sel({sig}, const bool want_jac,")
         L.append("      T* __restrict__ f1, A J)")
         L.append("  {")
-        L += ["    " + x for x in head + self._dev_fd_jacobian_lines(with_rhs=True, select=True)]
+        L += ["    " + x for x in head + self._dev_fd_jacobian_lines(select=True)]
         L.append("    (void)time; (void)P; (void)PD; (void)F; (void)f1; (void)J;")
         L.append("  }")
         L.append("")
@@ -881,7 +872,7 @@ class ModelSource:
         L.append(f"  __device__ static __forceinline__ void rhs2_fd_jacobian({sig}, const double t0,")
         L.append("      T* __restrict__ f0, T* __restrict__ f1, A J)")
         L.append("  {")
-        L += ["    " + x for x in head + self._dev_fd_jacobian_lines(with_rhs=True, with_t0=True)]
+        L += ["    " + x for x in head + self._dev_fd_jacobian_lines(with_t0=True)]
         L.append("    (void)time; (void)t0; (void)P; (void)PD; (void)F; (void)f0; (void)f1; (void)J;")
         L.append("  }")
         L.append("")
@@ -958,19 +949,12 @@ class ModelSource:
         L.append("  {")
         L += I4(lus.solve_lines("J", "b", "x"))
         L.append("  }")
-        L.append("  // forward differences: zero the entries outside the Jacobian's structure, then")
-        L.append("  // column i = (f2 - f1) / delta at its structural rows")
+        L.append("  // forward differences: zero the entries outside the Jacobian's structure")
         L.append("  template <class A>")
         L.append("  __device__ static __forceinline__ void fd_clear(A J)")
         L.append("  {")
         L += I4(lus.clear_extra_lines("J"))
         L.append("    (void)J;")
-        L.append("  }")
-        L.append("  template <class A>")
-        L.append("  __device__ static __forceinline__ void fd_column(const int i, const double* f1, const double* f2,")
-        L.append("                                                   const double delta, A J)")
-        L.append("  {")
-        L += I4(lus.fd_column_lines("J"))
         L.append("  }")
         L.append("  // dense row-major copy: out(r*n + c, value) for every entry")
         L.append("  template <typename T, class Out>")

@@ -15,6 +15,8 @@ _COST = ((r"gexp2?\(", 24), (r"glog\(", 40), (r"gsqrt\(", 20), (r"gpow\(", 64), 
 _DEFINITION = re.compile(r"const (?:T|double|bool) (\w+) = (.*);$")
 _OUTPUT = re.compile(r"\w+\[(\d+)\] = (.*);$")
 PARTS = 4
+# states of a model worth dealing out, and those the exchange buffers hold
+MIN_ROWS, MAX_ROWS = 9, 64
 
 
 def row_groups(lines: Sequence[str], rows: int, update: int) -> List[int]:

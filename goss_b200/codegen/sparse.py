@@ -113,18 +113,5 @@ class LUStructure:
         L += [f"{dst}[{d}] = {dst}[{d}] + 1.0 * 1.0;" for d in self.diag]
         return L
 
-    def fd_column_lines(self, J: str = "J") -> List[str]:
-        """``switch`` over column i storing ``(f2[r] - f1[r]) / delta`` at the
-        structural rows of that column."""
-        n, p = self.n, self.pos
-        L = ["switch (i) {"]
-        for c in range(n):
-            rows = [r for r in range(n) if self.jac[r][c]]
-            stores = " ".join(f"{J}[{p[(r, c)]}] = (f2[{r}] - f1[{r}]) / delta;" for r in rows)
-            L.append(f"case {c}: {stores} break;")
-        L.append("default: break;")
-        L.append("}")
-        return L
-
     def clear_extra_lines(self, J: str = "J") -> List[str]:
         return [f"{J}[{k}] = 0.0;" for k in self.extra]

@@ -1022,8 +1022,8 @@ __global__ void __launch_bounds__(128, 2) group_kernel(const __grid_constant__ E
     }
 }
 
-// Models generated without row groups, with too few states to share out (or too
-// many for the exchange buffers) keep a thread per node.  So does GRL2: a copy
+// Models generated without row groups (too few states to share out, or too many
+// for the exchange buffers) keep a thread per node.  So does GRL2: a copy
 // of the program that leaves out rows contracts other products, and over 100 ms
 // of 2,048 nodes GRL2 carried that to 1.6e-9 of the reference (bar 1e-9).
 template <class M, class = void>
@@ -1032,7 +1032,7 @@ struct HasRowGroups {
 };
 template <class M>
 struct HasRowGroups<M, decltype(void(M::linear_group(0) + M::rhs_group(0)))> {
-    static constexpr bool value = M::num_states > 8 && M::num_states <= 64;
+    static constexpr bool value = true;
 };
 template <class M, typename T, Explicit S>
 constexpr bool explicit_groups =

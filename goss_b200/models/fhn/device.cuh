@@ -65,22 +65,11 @@ struct M_fhn {
     x[1] = x[1] / J[3];
     { double s = 0.0; s = s + J[1] * x[1]; x[0] = (x[0] - s) / J[0]; }
   }
-  // forward differences: zero the entries outside the Jacobian's structure, then
-  // column i = (f2 - f1) / delta at its structural rows
+  // forward differences: zero the entries outside the Jacobian's structure
   template <class A>
   __device__ static __forceinline__ void fd_clear(A J)
   {
     (void)J;
-  }
-  template <class A>
-  __device__ static __forceinline__ void fd_column(const int i, const double* f1, const double* f2,
-                                                   const double delta, A J)
-  {
-    switch (i) {
-    case 0: J[0] = (f2[0] - f1[0]) / delta; J[2] = (f2[1] - f1[1]) / delta; break;
-    case 1: J[1] = (f2[0] - f1[0]) / delta; J[3] = (f2[1] - f1[1]) / delta; break;
-    default: break;
-    }
   }
   // dense row-major copy: out(r*n + c, value) for every entry
   template <typename T, class Out>
@@ -156,38 +145,9 @@ struct M_fhn {
     (void)time; (void)P; (void)PD; (void)F;
   }
 
-  // the rows of linearized_split and of rhs_split dealt to the four warps of a block
-  __host__ __device__ static constexpr int linear_group(int i) { return "01"[i] - '0'; }
-  __host__ __device__ static constexpr int rhs_group(int i) { return "01"[i] - '0'; }
-
   // forward-difference Jacobian of rhs_split at y into the packed Newton matrix (structural
-  // entries; fd_clear sets the others): f1 = f(y, time); column i recomputes only the
-  // statements of its rows that depend on state i
-  template <typename T, class A>
-  __device__ static __forceinline__ void fd_jacobian(const T* __restrict__ y, const double time, const T* __restrict__ P, const double* __restrict__ PD, const T* __restrict__ F, const T* __restrict__ f1, A J)
-  {
-    const T s_v = y[0];
-    const T s_s = y[1];
-    const T v_I = ((P[11] + s_v)*((P[12]*s_s) + (P[14]*(P[13] + s_v)*(P[9] - ((s_v))))));
-    const double v_i_Stim = (PD[5]*(1.0 - ((1.0/(1.0 + exp((PD[16] + (5.0*time)))))))/(1.0 + exp((PD[15] + (5.0*time)))));
-    {
-      const double d = sqrt(1e-15 * (1e-5 > fabs(double(y[0])) ? 1e-5 : fabs(double(y[0]))));
-      const T v___yp0 = T(double(y[0]) + d);
-      const T v_I__k0 = ((v___yp0 + P[11])*((P[12]*s_s) + (P[14]*(v___yp0 + P[13])*(P[9] - ((v___yp0))))));
-      J[0] = (((v_I__k0 + T(v_i_Stim))) - f1[0]) / d;
-      J[2] = (((P[1]*(v___yp0 + P[11] + (P[17]*s_s)))) - f1[1]) / d;
-    }
-    {
-      const double d = sqrt(1e-15 * (1e-5 > fabs(double(y[1])) ? 1e-5 : fabs(double(y[1]))));
-      const T v___yp1 = T(double(y[1]) + d);
-      const T v_I__k1 = ((P[11] + s_v)*((v___yp1*P[12]) + (P[14]*(P[13] + s_v)*(P[9] - ((s_v))))));
-      J[1] = (((v_I__k1 + T(v_i_Stim))) - f1[0]) / d;
-      J[3] = (((P[1]*(P[11] + s_v + (v___yp1*P[17])))) - f1[1]) / d;
-    }
-    (void)time; (void)P; (void)PD; (void)F; (void)f1; (void)J;
-  }
-
-  // the same, also writing f1 = f(y, time) (rhs_split) from its unperturbed statements
+  // entries; fd_clear sets the others); column i recomputes only the statements of its rows
+  // that depend on state i.  f1 = f(y, time) (rhs_split) from the unperturbed statements
   template <typename T, class A>
   __device__ static __forceinline__ void rhs_fd_jacobian(const T* __restrict__ y, const double time, const T* __restrict__ P, const double* __restrict__ PD, const T* __restrict__ F, T* __restrict__ f1, A J)
   {

@@ -63,24 +63,13 @@ struct M_oscilator__5dc98ee0 {
     x[1] = x[1] / J[3];
     { double s = 0.0; s = s + J[1] * x[1]; x[0] = (x[0] - s) / J[0]; }
   }
-  // forward differences: zero the entries outside the Jacobian's structure, then
-  // column i = (f2 - f1) / delta at its structural rows
+  // forward differences: zero the entries outside the Jacobian's structure
   template <class A>
   __device__ static __forceinline__ void fd_clear(A J)
   {
     J[0] = 0.0;
     J[3] = 0.0;
     (void)J;
-  }
-  template <class A>
-  __device__ static __forceinline__ void fd_column(const int i, const double* f1, const double* f2,
-                                                   const double delta, A J)
-  {
-    switch (i) {
-    case 0: J[2] = (f2[1] - f1[1]) / delta; break;
-    case 1: J[1] = (f2[0] - f1[0]) / delta; break;
-    default: break;
-    }
   }
   // dense row-major copy: out(r*n + c, value) for every entry
   template <typename T, class Out>
@@ -137,32 +126,9 @@ struct M_oscilator__5dc98ee0 {
     (void)time; (void)P; (void)PD; (void)F;
   }
 
-  // the rows of linearized_split and of rhs_split dealt to the four warps of a block
-  __host__ __device__ static constexpr int linear_group(int i) { return "01"[i] - '0'; }
-  __host__ __device__ static constexpr int rhs_group(int i) { return "01"[i] - '0'; }
-
   // forward-difference Jacobian of rhs_split at y into the packed Newton matrix (structural
-  // entries; fd_clear sets the others): f1 = f(y, time); column i recomputes only the
-  // statements of its rows that depend on state i
-  template <typename T, class A>
-  __device__ static __forceinline__ void fd_jacobian(const T* __restrict__ y, const double time, const T* __restrict__ P, const double* __restrict__ PD, const T* __restrict__ F, const T* __restrict__ f1, A J)
-  {
-    const T s_x = y[0];
-    const T s_y = y[1];
-    {
-      const double d = sqrt(1e-15 * (1e-5 > fabs(double(y[0])) ? 1e-5 : fabs(double(y[0]))));
-      const T v___yp0 = T(double(y[0]) + d);
-      J[2] = (((v___yp0*F[1])) - f1[1]) / d;
-    }
-    {
-      const double d = sqrt(1e-15 * (1e-5 > fabs(double(y[1])) ? 1e-5 : fabs(double(y[1]))));
-      const T v___yp1 = T(double(y[1]) + d);
-      J[1] = (((-(v___yp1*F[0]))) - f1[0]) / d;
-    }
-    (void)time; (void)P; (void)PD; (void)F; (void)f1; (void)J;
-  }
-
-  // the same, also writing f1 = f(y, time) (rhs_split) from its unperturbed statements
+  // entries; fd_clear sets the others); column i recomputes only the statements of its rows
+  // that depend on state i.  f1 = f(y, time) (rhs_split) from the unperturbed statements
   template <typename T, class A>
   __device__ static __forceinline__ void rhs_fd_jacobian(const T* __restrict__ y, const double time, const T* __restrict__ P, const double* __restrict__ PD, const T* __restrict__ F, T* __restrict__ f1, A J)
   {

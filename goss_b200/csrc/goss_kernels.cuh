@@ -1282,8 +1282,7 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
             // refactorise, its f(y, tn) evaluation writes f(y, t) as well
             prev_pending = false;
             if (!IE && fabs(sp.theta - 1.0) > kGossEps) {
-                if (one_eval32 || (!(relative_residual < sp.relative_tolerance) &&
-                                   (recompute || always))) {
+                if (!(relative_residual < sp.relative_tolerance) && (recompute || always)) {
                     prev_pending = true;
                 } else {
                     rhs64<M>(y, t, a.P, F, f1);
@@ -1303,20 +1302,7 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
         // or the statements the analytic Jacobian shares with f
         if constexpr (one_eval32) {
             const bool want_jac = !(relative_residual < sp.relative_tolerance) && (recompute || always);
-            // at a step's first iteration (yz = y) f(y, t) for the explicit part, then f(yz, tn)
-#pragma unroll 1
-            for (int k = (!IE && prev_pending) ? 0 : 1; k < 2; ++k) {
-                double g[n];
-                rhs64<M>(yz, k == 0 ? t : tn, a.P, F, g);
-#pragma unroll
-                for (int i = 0; i < n; ++i) {
-                    if (k == 0)
-                        prev[i] = (1 - sp.theta) * g[i];
-                    else
-                        f1[i] = g[i];
-                }
-            }
-            prev_pending = false;
+            rhs64<M>(yz, tn, a.P, F, f1);
             if (want_jac)
                 jacobian32<M>(yz, tn, a.P32, a.P, F, J);
         } else if constexpr (one_eval) {
@@ -1331,7 +1317,7 @@ __global__ void __launch_bounds__(GOSS_THETA_THREADS, GOSS_THETA_MIN_BLOCKS)
         } else if (!(relative_residual < sp.relative_tolerance) && (recompute || always)) {
             if constexpr (J32) {
                 // FP64 right-hand sides, the FP32 Jacobian
-                if (!IE && prev_pending) {
+                if (prev_pending) {
                     rhs64<M>(yz, t, a.P, F, b);
                     for (int i = 0; i < n; ++i)
                         prev[i] = (1 - sp.theta) * b[i];

@@ -101,17 +101,33 @@ class SolverTrace:
         self._checkpoints = torch.zeros((self.num_checkpoints, rows, self.ld), dtype=cp_dtype, device=dev)
         sld = (self.N + 255) // 256 * 256 + 256
         segment_bytes = self.K * self.n * sld * cp_dtype.itemsize
-        # RK4 in double precision: room for three stage derivatives of every
-        # step beside its input while that stays small
-        self._keep_stages = (solver == "RK4" and self.precision == _capi.GOSS_FP64
-                             and 4 * segment_bytes <= _STAGE_SCRATCH_BYTES)
-        self._scratch = torch.zeros((self.K, 4 * self.n if self._keep_stages else self.n, sld), dtype=cp_dtype,
-                                    device=dev)
-        if tape_bytes == "auto":
-            tape_bytes = torch.cuda.mem_get_info(dev)[0] - int(tape_reserve)
+        auto = isinstance(tape_bytes, str) and tape_bytes == "auto"
+        if auto:  # what is left beside the scratch and the reserve
+            tape_bytes = torch.cuda.mem_get_info(dev)[0] - segment_bytes - int(tape_reserve)
         elif not isinstance(tape_bytes, numbers.Integral) or isinstance(tape_bytes, bool):
             raise TypeError("tape_bytes must be an int or 'auto'")
-        self.taped_segments = int(min(self.num_checkpoints, max(0, int(tape_bytes)) // segment_bytes))
+
+        def segments(nbytes):
+            return int(min(self.num_checkpoints, max(0, int(nbytes)) // segment_bytes))
+
+        self.taped_segments = segments(tape_bytes)
+        # RK4 in double precision: where segments are recomputed, room for three
+        # stage derivatives of every step beside its input while that stays
+        # small.  It saves a recomputed segment as much as a tape saves, so with
+        # "auto" the tape leaves that room.
+        self._keep_stages = (solver == "RK4" and self.precision == _capi.GOSS_FP64
+                             and self.taped_segments < self.num_checkpoints
+                             and 4 * segment_bytes <= _STAGE_SCRATCH_BYTES)
+        if self._keep_stages and auto:
+            self.taped_segments = segments(tape_bytes - 3 * segment_bytes)
+        try:  # every row is written before it is read
+            self._scratch = torch.empty((self.K, 4 * self.n if self._keep_stages else self.n, sld), dtype=cp_dtype,
+                                        device=dev)
+        except torch.OutOfMemoryError:
+            if not self._keep_stages:
+                raise
+            self._keep_stages = False
+            self._scratch = torch.empty((self.K, self.n, sld), dtype=cp_dtype, device=dev)
         self._tape = (torch.empty((self.taped_segments, self.K, self.n, sld), dtype=cp_dtype, device=dev)
                       if self.taped_segments else None)
         self._states = torch.zeros((self.n, self.ld), dtype=torch.float64, device=dev)
@@ -148,7 +164,7 @@ class SolverTrace:
         L.trace = self._trace.data_ptr()
         L.trace_bar = trace_bar.data_ptr() if trace_bar is not None else None
         L.scratch = self._scratch.data_ptr()
-        L.keep_stages = self._keep_stages and self.taped_segments < self.num_checkpoints
+        L.keep_stages = self._keep_stages
         L.field_params_bar = fp_bar.data_ptr() if fp_bar is not None else None
         L.states_bar = states_bar.data_ptr() if states_bar is not None else None
         L.flags = self._flags.data_ptr()

@@ -198,7 +198,7 @@ struct AdjointArgs {
     void* checkpoints;         // [C][2n][ld] float (FP32: hi, lo) or [C][n][ld] double
     double* trace;             // [J][ld]
     const double* trace_bar;   // [J][ld]
-    T* scratch;                // [K][n][sld], sld = num_nodes rounded up to 256, plus 256
+    T* scratch;                // [K][n][sld] ([K][4 n][sld] with keep_stages), sld = num_nodes rounded up to 256, plus 256
     T* tape;                   // [taped_segments][K][n][sld]: step inputs of the last segments
     double* fparams_bar;       // [nfp][ld]
     double* states_bar;        // [n][ld]

@@ -288,8 +288,9 @@ struct Acc<float> {
 
 // renormalize() of all states.  FP32: the same operations on pairs of states in
 // packed arithmetic, with one range check for all of them instead of one branch
-// per state; where a sum is outside the range (zero, tiny, not finite) every
-// state takes the scalar form.  A one-step forward of a cardiac model spends
+// per state; where a sum is outside the range (zero, tiny, infinite) every
+// state takes the scalar form.  The check does not see a NaN, which passes
+// through the packed form as a NaN and leaves its pair's other state alone.  A one-step forward of a cardiac model spends
 // about as many instructions here as in its update, and the batch kernel is
 // bound by issuing them: 492,003 nodes of three models x 100 forwards 2.28 -> 1.94 ms.
 template <int n>

@@ -5,7 +5,8 @@
 //                       steps, GRL1.cpp:61-82 / RK4.cpp:68-102)
 // storing the traced state after every interval (the trace) and the full
 // state every K internal steps (checkpoints; K a multiple of S).  Each step
-// is explicit_step of goss_kernels.cuh, the solver kernels' own arithmetic.
+// is explicit_step of goss_kernels.cuh, the arithmetic of the solver kernels with
+// a thread per node.
 //
 // Backward (adjoint_kernel): given the cotangent of the trace, walk the
 // checkpoint segments from last to first; recompute each segment's K states

@@ -484,8 +484,10 @@ struct KeepNothing {
 };
 
 // One internal step of an explicit solver at time lt with step ldt, in place
-// on the accumulated states (shared by the solver kernels and the adjoint
-// kernels' record and recompute passes, so all take identical arithmetic).
+// on the accumulated states (shared by the thread-per-node solver kernels, the
+// batch kernel and the adjoint kernels' record and recompute passes, so all take
+// identical arithmetic; FP64 GRL1 on few nodes goes by group_step, which differs
+// by rounding).
 // keep(stage, k) sees RK4's stage derivatives.
 template <class M, typename T, Explicit S, class Keep = KeepNothing>
 __device__ __forceinline__ void explicit_step(Acc<T>* y, const double lt, const double ldt, const T* __restrict__ P,
@@ -1940,7 +1942,8 @@ inline int launch_explicit(const goss_launch* L)
     const bool wide = explicit_two_shapes<T, S> && block == 128 && explicit_blocks<S>(grid) == 2;
     constexpr int wide_blocks = explicit_two_shapes<T, S> ? 2 : ExplicitMinBlocks<T>::value;
     if constexpr (explicit_groups<M, T, S>) {
-        if (block == 128 && explicit_in_groups(L->num_nodes, S == Explicit::GRL1 ? a.delta : 1.0)) {
+        // a block size of the user's keeps a thread per node whatever the system's size
+        if (!L->block && explicit_in_groups(L->num_nodes, S == Explicit::GRL1 ? a.delta : 1.0)) {
             group_kernel<M, S><<<(L->num_nodes + 31) / 32, 128, 0, st>>>(a);
             return cudaPeekAtLastError() == cudaSuccess ? 0 : GOSS_ERR_CUDA;
         }

@@ -98,8 +98,6 @@ typedef struct goss_solver_params {
     double theta;                   /* ThetaSolver.h:37 */
 } goss_solver_params;
 
-/* One kernel launch of a solver over a node range (filled by the runtime,
- * consumed by a model module's launch function). */
 /* One forward of a schedule: its start time, internal step and number of steps. */
 typedef struct goss_forward {
     double t;
@@ -107,6 +105,8 @@ typedef struct goss_forward {
     uint64_t nsteps;
 } goss_forward;
 
+/* One kernel launch of a solver over a node range (filled by the runtime,
+ * consumed by a model module's launch function). */
 typedef struct goss_launch {
     int32_t solver;
     int32_t precision;
@@ -357,7 +357,12 @@ GOSS_API uint32_t goss_system_num_nodes(const goss_system* sys);
 /* Launch configuration (threads per block, a multiple of 32; 0 = the default:
  * 128 for the explicit solvers, up to 256 by the number of nodes for the
  * implicit ones, whose blocks run in lockstep; the kernels take at most 128 and
- * 256). */
+ * 256).  With the default, FP64 GRL1 and RK4 systems of at most 16 nodes per SM
+ * (2,368 on 148 SMs) and of models with 9 to 64 states split a node's rows over
+ * the warps of a block.  RK4 gives the same bits either way; GRL1 differs by
+ * rounding (4e-10 of a state at most in runs through an upstroke), so a caller
+ * whose FP64 GRL1 results must not depend on the number of nodes, e.g. on how
+ * they are distributed, sets a block size. */
 GOSS_API int goss_system_set_block_size(goss_system* sys, uint32_t block);
 
 /* Status word accumulated since the last clear (goss_flag_bits). */

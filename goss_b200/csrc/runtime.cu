@@ -14,7 +14,9 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -1479,18 +1481,22 @@ int solve_scheduled(goss_system* s, double* field_states, const double* t, uint6
 {
     const uint64_t per = (uint64_t)s->N * s->fsi.size(), times = nt - 1;
     const uint64_t head = sizeof(goss_forward) / sizeof(double);
-    uint64_t chunk = std::min<uint64_t>(times, std::max<uint64_t>(1, (256ull << 20) / (8 * per)));
+    uint64_t chunk = std::min<uint64_t>(times, std::max<uint64_t>(1, (256ull << 20) / (8 * (per + head))));
     double* d_own = nullptr;
     double* d_buf = s->d_stage;
     const uint64_t staged = s->stage_elems / (per + head);
-    if (staged >= std::min<uint64_t>(chunk, 32)) {
+    const bool own = staged < std::min<uint64_t>(chunk, 32);
+    if (!own)
         chunk = std::min(chunk, staged);
-    } else {
+    const std::unique_ptr<goss_forward[]> schedule(new (std::nothrow) goss_forward[chunk]);
+    if (!schedule)
+        return fail(&s->last_error, GOSS_ERR_CUDA, "solve: no host memory for a schedule of %llu times",
+                    (unsigned long long)chunk);
+    if (own) {
         CUDA_TRY(s, cudaMalloc(&d_own, sizeof(double) * (per + head) * chunk));
         d_buf = d_own;
     }
     int rc = 0;
-    std::vector<goss_forward> schedule(chunk);
     for (uint64_t first = 0; first < times && !rc; first += chunk) {
         const uint64_t count = std::min(chunk, times - first);
         for (uint64_t k = 0; k < count; ++k) {
@@ -1505,7 +1511,7 @@ int solve_scheduled(goss_system* s, double* field_states, const double* t, uint6
         L.schedule = reinterpret_cast<const goss_forward*>(d_buf);
         L.out = d_buf + head * chunk;
         L.tangled = tangled;
-        cudaError_t e = cudaMemcpyAsync(d_buf, schedule.data(), sizeof(goss_forward) * count, cudaMemcpyHostToDevice,
+        cudaError_t e = cudaMemcpyAsync(d_buf, schedule.get(), sizeof(goss_forward) * count, cudaMemcpyHostToDevice,
                                         s->stream);
         if (e == cudaSuccess)
             rc = launch_forward(s, t[first], t[first + 1] - t[first], L);

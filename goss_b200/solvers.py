@@ -158,7 +158,12 @@ class ODESolver(abc.ABC):
         t = np.asarray(t, dtype=np.float64)
         y = np.zeros((t.size, self.num_states))
         y[0, :] = y0
-        if t.size > 1:
+        if type(self).forward is not ODESolver.forward:
+            cur = np.array(y0, dtype=np.float64)
+            for it in range(1, t.size):  # a subclass's own forward
+                self.forward(cur, t[it - 1], t[it] - t[it - 1])
+                y[it, :] = cur
+        elif t.size > 1:
             # every time enqueued at once, the states copied back together
             self._one_node()._solve_states(y[0], t, y)
         return y

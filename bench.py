@@ -944,7 +944,7 @@ def measured_peaks(dev):
 # GRL1> (split program): the thread-level dadd + dmul + dfma counts of one ncu
 # capture of `bench.py --profile double --steps 1 --warmup 1 --nodes 56832`
 # divided by the cell-steps of the launch (56,832 x 1000)
-FP64_PIPE_OPS_PER_CELL_STEP = 1737.0  # dadd 200 + dmul 437 + dfma 1100 (B200, ncu)
+FP64_PIPE_OPS_PER_CELL_STEP = 1884.0  # dadd 248 + dmul 363 + dfma 1273 (B200, ncu)
 
 
 def roofline_fp64(value_fp64, peaks):

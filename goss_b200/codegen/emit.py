@@ -797,7 +797,7 @@ class ModelSource:
         L.append("  }")
         L.append("")
         L.append("  // linearized with every distinct transcendental and reciprocal of a state-dependent")
-        L.append("  // operand evaluated once (the FP32 kernels' form; FP64 keeps the reference's operations)")
+        L.append("  // operand evaluated once")
         L.append("  template <typename T>")
         L.append(f"  __device__ static __forceinline__ void linearized_split({sig}, T* __restrict__ linear, T* __restrict__ rhs)")
         L.append("  {")

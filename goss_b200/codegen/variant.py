@@ -30,7 +30,7 @@ from .odeparse import ODEModel
 
 # of the generated text: a model compiled at run time is written again when it
 # was generated by another version
-GENERATOR_VERSION = "10"
+GENERATOR_VERSION = "11"
 # of the key below, which names a model and its choices
 _KEY_VERSION = "8"
 

@@ -1043,11 +1043,13 @@ constexpr bool explicit_groups =
 
 // Whether to split the rows: blocks of 32 nodes on at most half the SMs.  The
 // time is flat to a quarter of them, then grows by the block as the SMs of a
-// GPC fetch four instruction streams each through one cache.  TP06, 100 steps,
-// thread per node / split, ms (4 fields, FP64):
-//   nodes      256          1,184        1,792        2,368        3,840
-//   GRL1   1.00 / 0.203   1.05 / 0.226   1.05 / 0.338   1.09 / 0.404   1.04 / 0.595
-//   RK4   1.340 / 0.710  1.511 / 0.763  1.512 / 1.164  1.546 / 1.392  1.558 / 2.079
+// GPC fetch four instruction streams each through one cache.  100 steps, thread
+// per node / split, ms (4 fields, FP64; at 3,840 nodes TP06's RK4 takes 1.56 / 2.08):
+//   nodes          1            256          1,184         1,792         2,368
+//   TP06 GRL1  0.97 / 0.19   0.97 / 0.21   0.97 / 0.22   0.97 / 0.34   0.98 / 0.40
+//   TP06 RK4   1.42 / 0.62   1.34 / 0.70   1.50 / 0.76   1.50 / 1.17   1.56 / 1.39
+//   TT04 GRL1  0.88 / 0.17   0.88 / 0.19   0.88 / 0.21   0.88 / 0.32   0.88 / 0.38
+//   TT04 RK4   1.19 / 0.55   1.06 / 0.65   1.30 / 0.71   1.30 / 1.11   1.36 / 1.32
 // Coefficients within [-delta, delta] take the Euler increment; a delta below
 // kGrlTiny stays with the thread per node, whose division takes every operand.
 constexpr double kGrlTiny = 0x1p-1000;

@@ -116,7 +116,7 @@ struct M_fhn {
   }
 
   // linearized with every distinct transcendental and reciprocal of a state-dependent
-  // operand evaluated once (the FP32 kernels' form; FP64 keeps the reference's operations)
+  // operand evaluated once
   template <typename T>
   __device__ static __forceinline__ void linearized_split(const T* __restrict__ y, const double time, const T* __restrict__ P, const double* __restrict__ PD, const T* __restrict__ F, T* __restrict__ linear, T* __restrict__ rhs)
   {
